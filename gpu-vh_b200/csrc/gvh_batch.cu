@@ -134,6 +134,7 @@ template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
 __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS)
     batch_stage_kernel(EventDev *ev, const int *__restrict__ tile_event, const int *__restrict__ ntiles_p,
                        int tile_x) {
+  eos_table_load<EOS>();
   const int ntiles = *ntiles_p;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     EventDev &E = ev[tile_event[tile]];

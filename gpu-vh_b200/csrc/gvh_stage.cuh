@@ -131,19 +131,29 @@ __device__ __forceinline__ FaceSpeeds<double> face_speeds(const StageArgs &a, in
     cr[2 * kBlock] = q2 - D0 * 0.25;  // bwd qR
     cr[3 * kBlock] = q1 + Dm * 0.25;  // bwd qL
   }
+  // two recoveries at a time (energy_from_conserved_n)
   double w[4] = {0, 0, 0, 0};
+  bool bad = false;
 #pragma unroll 1
-  for (int h = 0; h < 4; ++h) {
-    double st[9][1];
+  for (int h = 0; h < 4; h += 2) {
+    double st[9][2];
 #pragma unroll
-    for (int r = 0; r < 9; ++r) st[r][0] = r < NR ? cache[(4 * r + h) * kBlock] : 0.0;
-    double w1[1];
-    inferred_face_n<EOS, 1>(a.t_euler, axis, st[0], st[1], st[2], st[3], st[4], st[5], st[6], st[7], st[8], g0, w1,
-                            status);
-    w[0] = h == 0 ? w1[0] : w[0];
-    w[1] = h == 1 ? w1[0] : w[1];
-    w[2] = h == 2 ? w1[0] : w[2];
-    w[3] = h == 3 ? w1[0] : w[3];
+    for (int r = 0; r < 9; ++r) {
+      st[r][0] = r < NR ? cache[(4 * r + h) * kBlock] : 0.0;
+      st[r][1] = r < NR ? cache[(4 * r + h + 1) * kBlock] : 0.0;
+    }
+    double w2[2];
+    inferred_face_n<EOS, 2>(a.t_euler, axis, st[0], st[1], st[2], st[3], st[4], st[5], st[6], st[7], st[8], g0, w2,
+                            bad);
+    w[0] = h == 0 ? w2[0] : w[0];
+    w[1] = h == 0 ? w2[1] : w[1];
+    w[2] = h == 2 ? w2[0] : w[2];
+    w[3] = h == 2 ? w2[1] : w[3];
+  }
+  if (__builtin_expect(bad, 0)) {
+    double v[4];
+    status |= face_velocities_general<EOS, NR>(a.t_euler, axis, cache, kBlock, g0.e, v);
+    w[0] = v[0]; w[1] = v[1]; w[2] = v[2]; w[3] = v[3];
   }
   FaceSpeeds<double> f;
   f.wRf = w[0]; f.wLf = w[1]; f.wRb = w[2]; f.wLb = w[3];
@@ -379,7 +389,7 @@ __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, in
 
 // The rest of a stage for one cell once out holds its Euler update: the Heun combination
 // (stage 2), primitive recovery at the new time, regulation, and the writes. Returns e.
-template <int EOS, bool SHEAR, bool BULK, bool STAGE2, int OSTRIDE>
+template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED, int OSTRIDE>
 __device__ __forceinline__ double stage_finish(const StageArgs &a, long long s, const double *out, const GuessEos &g0,
                                                unsigned status) {
   constexpr int NQ = NComp<SHEAR, BULK>::value;
@@ -394,7 +404,7 @@ __device__ __forceinline__ double stage_finish(const StageArgs &a, long long s, 
 
   // ---- primitive recovery at the new time (EnergyMomentumTensor.cu:110-154) ---------------
   const double tn = a.t_after;
-  Prim pr = inferred<EOS>(tn, o[0], o[1], o[2], o[3], SHEAR ? o[4] : 0.0, SHEAR ? o[5] : 0.0,
+  Prim pr = inferred<EOS, MIXED>(tn, o[0], o[1], o[2], o[3], SHEAR ? o[4] : 0.0, SHEAR ? o[5] : 0.0,
                           SHEAR ? o[6] : 0.0, SHEAR ? o[7] : 0.0, BULK ? o[NQ - 1] : 0.0, g0, status);
 
   // ---- regulation (RegulateDissipativeCurrents.cu:15-134) ----------------------------------
@@ -528,7 +538,7 @@ __device__ __forceinline__ double stage_cell_ijk(const StageArgs &a, int i, int 
     speed = fmax(speed, n_axis > 1 ? as * inv_spacing : 0.0);
   }
 
-  return stage_finish<EOS, SHEAR, BULK, STAGE2, kBlock>(a, s, out, g0, status);
+  return stage_finish<EOS, SHEAR, BULK, STAGE2, MIXED, kBlock>(a, s, out, g0, status);
 }
 
 // The cell with interior index id (i fastest).
@@ -556,6 +566,7 @@ inline dim3 stage_grid(long long ncells) { return dim3((unsigned)((ncells + kBlo
 // caller's dt.
 template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
 __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_kernel(const StageArgs a) {
+  eos_table_load<EOS>();
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double speed = 0.0;
   if (id < a.ncells) stage_cell<EOS, SHEAR, BULK, STAGE2, MIXED>(a, id, speed);
@@ -590,6 +601,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
   extern __shared__ double gvh_stage_smem[];
   double *out = gvh_stage_smem + threadIdx.x;
   double *cache = gvh_stage_smem + NQ * kBlock + threadIdx.x;
+  eos_table_load<EOS>();
   double speed = 0.0;
   bool live = id < a.ncells;
   int i = 0, j = 0, k = 0;
@@ -641,7 +653,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
 #pragma unroll
       for (int n = 0; n < NQ; ++n) out[n * kBlock] += inc[n * kBlock] * a.dt;
     }
-    stage_finish<EOS, SHEAR, BULK, STAGE2, kBlock>(a, s, out, guess_eos<EOS>(ePrev), status);
+    stage_finish<EOS, SHEAR, BULK, STAGE2, MIXED, kBlock>(a, s, out, guess_eos<EOS>(ePrev), status);
   }
   if (!STAGE2 && a.speed_max) {
     unsigned long long b = (unsigned long long)__double_as_longlong(fmax(speed, 0.0));
