@@ -4,13 +4,16 @@
 // with USE_APPROX_DERIVATIVE). Operation order follows the reference.
 #pragma once
 
+#include <type_traits>
+
 #include "gvh_physics.cuh"
 
 namespace gvh {
 
-// Division in the working precision: IEEE division in FP64 (the plain path follows the
-// reference to rounding), the fast reciprocal-based division in FP32 (mixed path).
-__device__ __forceinline__ double dv(double a, double b) { return a / b; }
+// Division in the working precision: reciprocal-based in both, to rounding in FP64 (div_fast;
+// the divisors here -- tau, u^tau, eta/s, the fits' denominators, zeta/s -- are normal numbers
+// in any state that is not already lost, and a NaN or an infinity stays one or becomes NaN).
+__device__ __forceinline__ double dv(double a, double b) { return div_fast(a, b); }
 __device__ __forceinline__ float dv(float a, float b) { return __fdividef(a, b); }
 
 // Flow state and limited first derivatives at a cell.
@@ -28,9 +31,10 @@ struct ShearT {
 
 // SourceTerms.cu:29-256. rhs[0..9] = d pi^{mu nu}/dtau (pitt..pinn), rhs[10] = dPi/dtau.
 // R = double reproduces the reference's FP64 arithmetic; R = float is the mixed path.
+// cs2_guess: c_s^2(e) from the cell's GuessEos (the FP64 path; the mixed path evaluates its own).
 template <int EOS, bool BULK, class R>
 __device__ __forceinline__ void pimunu_rhs(R *rhs, R t, R etabar, R e, R p, const CellFlowT<R> &f,
-                                           const ShearT<R> &pi, R Pi, R dkvk) {
+                                           const ShearT<R> &pi, R Pi, R dkvk, double cs2_guess) {
   const R ut = f.ut, ux = f.ux, uy = f.uy, un = f.un;
   const R pitt = pi.tt, pitx = pi.tx, pity = pi.ty, pitn = pi.tn, pixx = pi.xx, pixy = pi.xy, pixn = pi.xn;
   const R piyy = pi.yy, piyn = pi.yn, pinn = pi.nn;
@@ -169,7 +173,7 @@ __device__ __forceinline__ void pimunu_rhs(R *rhs, R t, R etabar, R e, R p, cons
   rhs[9] = dpinn * iut + pinn * dkvk;
   if (BULK) {
     // bulk coefficients (SourceTerms.cu:53-60, 238, 254)
-    R cs2 = sound_speed2<EOS>(e);
+    const R cs2 = std::is_same<R, double>::value ? R(cs2_guess) : sound_speed2<EOS>(e);
     R a = R(kF033) - cs2;
     R a2 = a * a;
     R beta_Pi = R(15.0) * a2 * (e + p);

@@ -97,16 +97,26 @@ struct FaceSpeeds {
 // :41-44) with the cell's own energy density as guess.
 // The half-cell states go to this thread's column of the shared-memory cache
 // (cache[(4 r + f) * kBlock]), from which phase B takes them instead of recomputing them.
+// The FP64 path also adds the terms of the axis's pi, Pi derivative sources (axis_pi_sources) that
+// the components passing through here give, from the neighbours already loaded: sink.
+struct PiSink {
+  double *out;            // the running update (or increments) of T^{tau mu}, kBlock apart
+  double v;               // u^axis / u^tau
+  double fac, dt;         // 1/(2 d), the time step (or 1)
+};
 template <int EOS, bool SHEAR, bool BULK, bool MIXED>
 __device__ __forceinline__ FaceSpeeds<double> face_speeds(const StageArgs &a, int s, int axis, const int (&o)[5],
-                                                       const GuessEos &g0, double *cache, unsigned &status) {
+                                                       const GuessEos &g0, const PiSink &sink, double *cache,
+                                                       unsigned &status) {
   // index f: 0 fwd R, 1 fwd L, 2 bwd R, 3 bwd L. The states go to the cache first; the four
   // recoveries then read them back one at a time (runtime loops keep the code small:
   // instruction fetch, not arithmetic, is what the long straight-line variant waited on).
   constexpr int NR = 4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0);
-  // three components per pass: their 15 stencil loads are in flight together (one at a time
-  // the loop waited on each component's loads; 3 measured 4% faster than 1, 2 and 9 slower)
-#pragma unroll 3
+  // three components per pass, or four where they divide without a rest: their 15 to 20 stencil
+  // loads are in flight together (of 9 components one at a time takes 1.324 ms per 131x131x61
+  // step, three 1.237, all 1.299; of 8, three 0.849, four 0.816)
+  constexpr int kPerPass = NR % 3 == 0 ? 3 : 4;
+#pragma unroll kPerPass
   for (int r = 0; r < NR; ++r) {
     const int c = (r < 8) ? r : 14;
     const double *q = a.qin + (size_t)c * a.cs + s;
@@ -124,6 +134,16 @@ __device__ __forceinline__ FaceSpeeds<double> face_speeds(const StageArgs &a, in
       Dm = limited_slope2(theta2, q0, q1, q2);
       D0 = limited_slope2(theta2, q1, q2, q3);
       Dp = limited_slope2(theta2, q2, q3, q4);
+    }
+    if (SHEAR && !MIXED && r >= 4) {
+      const double d = (q3 - q1) * sink.fac;
+      if (r < 8) {  // pi^{tau m}, m = r - 4
+        sink.out[(r - 4) * kBlock] += (d * sink.v) * sink.dt;
+        if (r == 5 + axis) sink.out[0] -= d * sink.dt;
+      } else {  // Pi
+        sink.out[0] -= (sink.v * d) * sink.dt;
+        sink.out[(1 + axis) * kBlock] -= (axis == 2 ? dv(d, a.t_euler * a.t_euler) : d) * sink.dt;
+      }
     }
     double *cr = cache + 4 * r * kBlock;
     cr[0] = q3 - Dp * 0.25;           // fwd qR
@@ -180,10 +200,13 @@ __device__ __forceinline__ R flux_from_states(R fR, R fL, R bR, R bL, const Face
   return -Hf + Hb;
 }
 
+// centred: the difference of the two neighbours, q(i+1) - q(i-1).
 template <class R>
-__device__ __forceinline__ R flux_difference(R theta, const double *q, const int (&o)[5], const FaceSpeeds<R> &f) {
+__device__ __forceinline__ R flux_difference(R theta, const double *q, const int (&o)[5], const FaceSpeeds<R> &f,
+                                             R &centred) {
   const R q0 = (R)__ldg(q + o[0]), q1 = (R)__ldg(q + o[1]), q2 = (R)__ldg(q), q3 = (R)__ldg(q + o[3]);
   const R q4 = (R)__ldg(q + o[4]);
+  centred = q3 - q1;
   const R theta2 = R(2) * theta;  // doubled slopes: q -+ D/2 = q -+ D2/4
   const R Dm = limited_slope2(theta2, q0, q1, q2);
   const R D0 = limited_slope2(theta2, q1, q2, q3);
@@ -192,6 +215,13 @@ __device__ __forceinline__ R flux_difference(R theta, const double *q, const int
   return flux_from_states<R>(q3 - Dp * qu, q2 + D0 * qu, q2 - D0 * qu, q1 + Dm * qu, f);
 }
 
+// The m with pi^{m axis} = component n (m = 0, 1, 2 for x, y, eta), or -1.
+__device__ __forceinline__ int spatial_of_pi(int n, int axis) {
+  // xx=8 xy=9 xn=10 yy=11 yn=12 nn=13
+  if (axis == 0) return n <= 10 ? n - 8 : -1;
+  if (axis == 1) return n == 9 ? 0 : n == 11 ? 1 : n == 12 ? 2 : -1;
+  return n == 10 ? 0 : n == 12 ? 1 : n == 13 ? 2 : -1;
+}
 // pi^{m a} component index for spatial m, a in {x, y, eta}.
 __device__ __forceinline__ int pi_spatial(int m, int a) {
   // xx=8 xy=9 xn=10 yy=11 yn=12 nn=13
@@ -204,7 +234,10 @@ __device__ __forceinline__ int pi_spatial(int m, int a) {
 //   S_0     = d(pi^{tt}) v - d(pi^{t a}) [- v d(Pi)]
 //   S_{m+1} = d(pi^{t m}) v - d(pi^{m a}) [- d(Pi), divided by tau^2 along eta, when m = a]
 // Sa: the axis's pi and Pi derivative sources of T^{tau mu} (SourceTerms.cu:443-567), in the
-// working precision; zero without shear.
+// working precision; zero without shear. The mixed path's form; the FP64 path adds the same terms
+// one by one where their stencils are loaded anyway (PiSink): 16 loads per axis and their
+// latency less, 131x131x61 step 1.260 -> 1.238 ms. (In FP32 the other order of the sum would
+// change the mixed path's results by its rounding, so it keeps this one.)
 template <bool SHEAR, bool BULK, class R>
 __device__ __forceinline__ void axis_pi_sources(const StageArgs &a, int s, int axis, const int (&o)[5], R inv_d,
                                                 const double *uc, R (&Sa)[4]) {
@@ -246,13 +279,21 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
   // Face states are recovered in FP64 on both paths (the mixed path rounds only the
   // resulting speeds): an FP32 recovery was tried and let a 2+1D hotspot event run away
   // to NaN that the FP64 recovery keeps finite.
-  const FaceSpeeds<double> fd = face_speeds<EOS, SHEAR, BULK, MIXED>(a, s, axis, o, g0, cache, status);
+  PiSink sink = {};
+  if (SHEAR && !MIXED) {
+    sink.out = out;
+    sink.v = dv(__ldg(a.uin + (1 + axis) * a.cs + s), __ldg(a.uin + s));
+    sink.fac = 0.5 * inv_spacing;
+    sink.dt = INCREMENT ? 1.0 : a.dt;
+    if (INCREMENT) out[0] = out[kBlock] = out[2 * kBlock] = out[3 * kBlock] = 0.0;
+  }
+  const FaceSpeeds<double> fd = face_speeds<EOS, SHEAR, BULK, MIXED>(a, s, axis, o, g0, sink, cache, status);
   FaceSpeeds<R> f;
   f.wRf = (R)fd.wRf; f.wLf = (R)fd.wLf; f.wRb = (R)fd.wRb; f.wLb = (R)fd.wLb;
   f.af = (R)fd.af; f.ab = (R)fd.ab;
 
   R Sa[4];
-  axis_pi_sources<SHEAR, BULK, R>(a, s, axis, o, inv_d, uc, Sa);
+  if (MIXED) axis_pi_sources<SHEAR, BULK, R>(a, s, axis, o, inv_d, uc, Sa);
   const R th = (R)a.theta;
   // the root-find components from the cache
   constexpr int NRC = 4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0);
@@ -262,8 +303,9 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
     const double *c = cache + 4 * rc * kBlock;
     R r = flux_from_states<R>((R)c[0], (R)c[kBlock], (R)c[2 * kBlock], (R)c[3 * kBlock], f);
     r = r * half_inv_d;
-    if (SHEAR && n < 4) r += Sa[n];
-    if (INCREMENT) out[n * kBlock] = (double)r;
+    if (SHEAR && MIXED && n < 4) r += Sa[n];
+    if (INCREMENT && (!SHEAR || MIXED || n >= 4)) out[n * kBlock] = (double)r;
+    else if (INCREMENT) out[n * kBlock] += (double)r;
     else out[n * kBlock] += (double)r * a.dt;
   }
   // pi^{ij} from the lattice, two components' stencil loads in flight at once (2 measured
@@ -271,7 +313,12 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
   if (SHEAR) {
 #pragma unroll 2
     for (int n = 8; n < 14; ++n) {
-      R r = flux_difference<R>(th, a.qin + (size_t)n * a.cs + s, o, f);
+      R centred;
+      const R r = flux_difference<R>(th, a.qin + (size_t)n * a.cs + s, o, f, centred);
+      if (!MIXED) {
+        const int m = spatial_of_pi(n, axis);
+        if (m >= 0) out[(1 + m) * kBlock] -= ((double)centred * sink.fac) * sink.dt;
+      }
       if (INCREMENT) out[n * kBlock] = (double)(r * half_inv_d);
       else out[n * kBlock] += (double)(r * half_inv_d) * a.dt;
     }
@@ -300,7 +347,7 @@ constexpr size_t stage_smem_bytes() {
 // (EulerStep.cu:946-1009, SourceTerms.cu:569-755).
 template <int EOS, bool SHEAR, bool BULK, bool MIXED, int OSTRIDE>
 __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, int i, int j, int k, double ePrev,
-                                             const double (&uc)[4], double *out) {
+                                             const double (&uc)[4], const GuessEos &g0, double *out) {
   using R = typename std::conditional<MIXED, float, double>::type;
   constexpr int NQ = NComp<SHEAR, BULK>::value;
   R q[NQ];
@@ -375,7 +422,7 @@ __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, in
   if (SHEAR) {
     ShearT<R> pi{q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13]};
     R rhs[11];
-    pimunu_rhs<EOS, BULK, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk);
+    pimunu_rhs<EOS, BULK, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk, g0.cs2);
 #pragma unroll
     for (int n = 4; n < NQ; ++n) S[n] = rhs[n - 4];
   }
@@ -513,10 +560,10 @@ __device__ __forceinline__ double stage_cell_ijk(const StageArgs &a, int i, int 
   double *out = gvh_stage_smem + threadIdx.x;
   double *cache = gvh_stage_smem + NQ * kBlock + threadIdx.x;
 
-  stage_source<EOS, SHEAR, BULK, MIXED, kBlock>(a, s, i, j, k, ePrev, uc, out);
+  const GuessEos g0 = guess_eos<EOS>(ePrev);
+  stage_source<EOS, SHEAR, BULK, MIXED, kBlock>(a, s, i, j, k, ePrev, uc, g0, out);
 
   // ---- flux divergence along x, y, eta (EulerStep.cu:1011-1277) -------------------------
-  const GuessEos g0 = guess_eos<EOS>(ePrev);
   speed = 0.0;
 #pragma unroll 1
   for (int axis = 0; axis < 3; ++axis) {
@@ -626,7 +673,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
 #pragma unroll
     for (int m = 0; m < 4; ++m) uc[m] = __ldg(a.uin + m * a.cs + s);
     if (part == 0) {
-      stage_source<EOS, SHEAR, BULK, MIXED, kBlock>(a, s, i, j, k, ePrev, uc, out);
+      stage_source<EOS, SHEAR, BULK, MIXED, kBlock>(a, s, i, j, k, ePrev, uc, guess_eos<EOS>(ePrev), out);
     } else {
       const int axis = part - 1;
       const int idx = axis == 0 ? i : axis == 1 ? j : k;
