@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS)
     batch_stage_kernel(EventDev *ev, const int *__restrict__ tile_event, const int *__restrict__ ntiles_p,
                        int tile_x) {
   eos_table_load<EOS>();
+  griddep_begin();
   const int ntiles = *ntiles_p;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     EventDev &E = ev[tile_event[tile]];
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS)
 // After stage 2: advance time, rotate the u buffers (u^{n+1} current, u^n previous, as the
 // reference's swapFluidVelocity), freeze-out bookkeeping.
 __global__ void batch_finish_kernel(EventDev *ev, int nslots) {
+  griddep_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots) return;
   EventDev &E = ev[i];
@@ -387,11 +389,11 @@ int launch_step_t(gvh_batch *b) {
   // events); otherwise a persistent grid of that many blocks
   const int g = b->grid > 0 ? b->grid : (b->ntiles > 0 ? b->ntiles : 1);
   const size_t smem = stage_smem_bytes<SHEAR, BULK>();
-  batch_stage_kernel<EOS, SHEAR, BULK, false, MIXED><<<g, kBlock, smem, b->stream>>>(b->d_ev, b->d_tile_event,
-                                                                                     b->d_ntiles, b->tile_x);
-  batch_stage_kernel<EOS, SHEAR, BULK, true, MIXED><<<g, kBlock, smem, b->stream>>>(b->d_ev, b->d_tile_event,
-                                                                                    b->d_ntiles, b->tile_x);
-  batch_finish_kernel<<<(kMaxEvents + 127) / 128, 128, 0, b->stream>>>(b->d_ev, kMaxEvents);
+  launch_overlapped(batch_stage_kernel<EOS, SHEAR, BULK, false, MIXED>, dim3(g), kBlock, smem, b->stream, b->d_ev,
+                    b->d_tile_event, b->d_ntiles, b->tile_x);
+  launch_overlapped(batch_stage_kernel<EOS, SHEAR, BULK, true, MIXED>, dim3(g), kBlock, smem, b->stream, b->d_ev,
+                    b->d_tile_event, b->d_ntiles, b->tile_x);
+  launch_overlapped(batch_finish_kernel, dim3((kMaxEvents + 127) / 128), 128, 0, b->stream, b->d_ev, kMaxEvents);
   BCUDA(cudaGetLastError());
   return GVH_OK;
 }

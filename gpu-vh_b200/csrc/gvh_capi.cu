@@ -26,6 +26,7 @@
 #include "gvh_layout.cuh"
 #include "gvh_nvtx.h"
 #include "gvh_stage.cuh"
+#include "gvh_stage_launch.h"
 #include "gvh_validity.cuh"
 
 using namespace gvh;
@@ -50,47 +51,14 @@ int fail(int code, const char *fmt, ...) {
     if (err_ != cudaSuccess) return fail(GVH_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(err_)); \
   } while (0)
 
-constexpr int kThreads = gvh::kBlock;
-
 }  // namespace
 
 
 namespace {
 
-template <int EOS, bool SHEAR, bool BULK, bool MIXED>
-int launch_stage_p(const gvh_handle *h, const StageArgs &a, bool stage2) {
-  const size_t smem = stage_smem_bytes<SHEAR, BULK>();
-  if (h->ncells < h->split_below) {
-    // fewer cells than one wave of the one-thread-per-cell kernel: four warps per 32 cells
-    const dim3 grid = split_grid(h->ncells);
-    if (stage2) kt_stage_split_kernel<EOS, SHEAR, BULK, true, MIXED><<<grid, kThreads, smem, h->stream>>>(a);
-    else kt_stage_split_kernel<EOS, SHEAR, BULK, false, MIXED><<<grid, kThreads, smem, h->stream>>>(a);
-    GVH_CUDA(cudaGetLastError());
-    return GVH_OK;
-  }
-  const dim3 grid = stage_grid(h->ncells);
-  if (stage2) kt_stage_kernel<EOS, SHEAR, BULK, true, MIXED><<<grid, kThreads, smem, h->stream>>>(a);
-  else kt_stage_kernel<EOS, SHEAR, BULK, false, MIXED><<<grid, kThreads, smem, h->stream>>>(a);
-  GVH_CUDA(cudaGetLastError());
-  return GVH_OK;
-}
-
-template <int EOS, bool SHEAR, bool BULK>
-int launch_stage(const gvh_handle *h, const StageArgs &a, bool stage2) {
-  if (h->precision == GVH_PRECISION_MIXED) return launch_stage_p<EOS, SHEAR, BULK, true>(h, a, stage2);
-  return launch_stage_p<EOS, SHEAR, BULK, false>(h, a, stage2);
-}
-
-template <int EOS>
-int dispatch_physics(const gvh_handle *h, const StageArgs &a, bool stage2) {
-  if (!h->shear) return launch_stage<EOS, false, false>(h, a, stage2);
-  if (!h->bulk) return launch_stage<EOS, true, false>(h, a, stage2);
-  return launch_stage<EOS, true, true>(h, a, stage2);
-}
-
 int dispatch(const gvh_handle *h, const StageArgs &a, bool stage2) {
-  if (h->eos == GVH_EOS_CONFORMAL) return dispatch_physics<EOS_CONFORMAL>(h, a, stage2);
-  return dispatch_physics<EOS_QCD>(h, a, stage2);
+  GVH_CUDA(launch_stage(h->eos, h->shear, h->bulk, h->precision, a, stage2, h->wave_cells, h->stream));
+  return GVH_OK;
 }
 
 // checkValidity after the step (FullyDiscreteKurganovTadmorScheme.cu:137): t + dt, the new
@@ -251,8 +219,7 @@ int gvh_create(const gvh_lattice_params *L, const gvh_hydro_params *H, const gvh
     static unsigned long long prepared = 0;
     std::lock_guard<std::mutex> lock(mu);
     if (dev < 64 && !(prepared & (1ull << dev))) {
-      GVH_CUDA(allow_all_stage_kernels());
-      GVH_CUDA(allow_all_split_kernels());
+      GVH_CUDA(prepare_stage_kernels());
       prepared |= 1ull << dev;
     }
   }
@@ -275,8 +242,7 @@ int gvh_create(const gvh_lattice_params *L, const gvh_hydro_params *H, const gvh
   h->theta = o.theta;
   h->cartesian = o.coordinates == GVH_COORDINATES_CARTESIAN;
   h->eos = o.eos; h->shear = o.shear; h->bulk = o.bulk; h->precision = o.precision; h->device = dev;
-  // one wave of the one-thread-per-cell stage kernel: below it the split kernel runs
-  h->split_below = (long long)sms * GVH_MIN_BLOCKS * kThreads;
+  h->wave_cells = stage_wave_cells(sms);
   h->ucur = 0; h->uprev = 1; h->ufree = 2;
 
   size_t nbuf = 2 * (size_t)h->nq + 3 + 12;

@@ -34,6 +34,7 @@
 #include "../../include/gvh.h"
 #include "gvh_physics.cuh"
 #include "gvh_stage.cuh"
+#include "gvh_stage_launch.h"
 
 using namespace gvh;
 
@@ -72,7 +73,7 @@ int scratch_address(int dev, unsigned char **out) {
       if (err != cudaSuccess)
         return nfail(GVH_ERR_CUDA, "cudaGetSymbolAddress(scratch) on device %d: %s", dev, cudaGetErrorString(err));
       // the stage kernels' shared-memory limit, part of the same one-time set-up
-      err = allow_all_stage_kernels();
+      err = prepare_stage_kernels();
       if (err != cudaSuccess)
         return nfail(GVH_ERR_CUDA, "stage kernel set-up on device %d: %s", dev, cudaGetErrorString(err));
       g_scratch_ptr[dev].store(p, std::memory_order_release);
@@ -90,21 +91,6 @@ struct DeviceRestore {
     if (saved >= 0) cudaSetDevice(saved);
   }
 };
-
-template <int EOS, bool SHEAR, bool BULK, bool MIXED>
-void launch_pair(const StageArgs &a1, const StageArgs &a2, long long, cudaStream_t st) {
-  const dim3 grid = stage_grid(a1.ncells);
-  const size_t smem = stage_smem_bytes<SHEAR, BULK>();
-  kt_stage_kernel<EOS, SHEAR, BULK, false, MIXED><<<grid, kBlock, smem, st>>>(a1);
-  kt_stage_kernel<EOS, SHEAR, BULK, true, MIXED><<<grid, kBlock, smem, st>>>(a2);
-}
-
-template <int EOS, bool MIXED>
-void dispatch_physics(int shear, int bulk, const StageArgs &a1, const StageArgs &a2, long long n, cudaStream_t st) {
-  if (!shear) launch_pair<EOS, false, false, MIXED>(a1, a2, n, st);
-  else if (!bulk) launch_pair<EOS, true, false, MIXED>(a1, a2, n, st);
-  else launch_pair<EOS, true, true, MIXED>(a1, a2, n, st);
-}
 
 }  // namespace
 
@@ -193,15 +179,8 @@ int gvh_rk2_step_noalloc(const gvh_lattice_params *L, const gvh_hydro_params *H,
   a2.qin = qS; a2.qn = q; a2.qout = q;
   a2.pin = pS; a2.pout = p;
   a2.uin = uS; a2.uprev = u; a2.uout = u_next;
-  const bool mixed = o.precision == GVH_PRECISION_MIXED;
-  if (o.eos == GVH_EOS_CONFORMAL) {
-    if (mixed) dispatch_physics<EOS_CONFORMAL, true>(o.shear, o.bulk, a1, a2, n, st);
-    else dispatch_physics<EOS_CONFORMAL, false>(o.shear, o.bulk, a1, a2, n, st);
-  } else {
-    if (mixed) dispatch_physics<EOS_QCD, true>(o.shear, o.bulk, a1, a2, n, st);
-    else dispatch_physics<EOS_QCD, false>(o.shear, o.bulk, a1, a2, n, st);
-  }
-  err = cudaGetLastError();
+  err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a1, false, 0, st);
+  if (err == cudaSuccess) err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a2, true, 0, st);
   if (err != cudaSuccess) return nfail(GVH_ERR_CUDA, "stage launch: %s", cudaGetErrorString(err));
   if (status_out) {
     err = cudaMemcpyAsync(status_out, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);

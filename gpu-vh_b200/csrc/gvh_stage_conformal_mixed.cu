@@ -1,0 +1,11 @@
+// gvh_stage_conformal_mixed.cu -- the stage kernels of the conformal equation of state, mixed precision.
+#include "gvh_stage_launch.cuh"
+
+namespace gvh {
+
+cudaError_t prepare_conformal_mixed() { return prepare_stages_of<EOS_CONFORMAL, true>(); }
+cudaError_t launch_conformal_mixed(const StageArgs &a, int shear, int bulk, bool stage2, long long wave, cudaStream_t st) {
+  return launch_stage_of<EOS_CONFORMAL, true>(a, shear, bulk, stage2, wave, st);
+}
+
+}  // namespace gvh

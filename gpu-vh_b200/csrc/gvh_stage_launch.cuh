@@ -1,0 +1,59 @@
+// gvh_stage_launch.cuh -- the body of a gvh_stage_*.cu: the stage kernels of one equation of state
+// and precision, and which of them a lattice takes.
+#pragma once
+
+#include "gvh_stage.cuh"
+#include "gvh_stage_launch.h"
+
+namespace gvh {
+
+// A lattice smaller than one wave of the one-thread-per-cell kernel (75,776 cells on 148 SMs) takes
+// four threads per cell: 33x33x17 conformal 49.9 -> 28.7 us per step, 61x61x1 QCD 56.3 -> 32.8;
+// a lattice that fills the GPU loses by it (131x131x61: 1.44 -> 2.14 ms).
+inline int stage_parts(long long ncells, long long wave) { return ncells < wave ? 4 : 1; }
+
+template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
+void launch_stage_kernel(const StageArgs &a, int parts, cudaStream_t st) {
+  const size_t smem = stage_smem_bytes<SHEAR, BULK>();
+  if (parts == 4)
+    launch_overlapped(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, split_grid(a.ncells, 4), kBlock, smem,
+                      st, a);
+  else
+    launch_overlapped(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, stage_grid(a.ncells), kBlock, smem, st, a);
+}
+
+template <int EOS, bool SHEAR, bool BULK, bool MIXED>
+void launch_stage_physics(const StageArgs &a, bool stage2, int parts, cudaStream_t st) {
+  if (stage2) launch_stage_kernel<EOS, SHEAR, BULK, true, MIXED>(a, parts, st);
+  else launch_stage_kernel<EOS, SHEAR, BULK, false, MIXED>(a, parts, st);
+}
+
+template <int EOS, bool MIXED>
+cudaError_t launch_stage_of(const StageArgs &a, int shear, int bulk, bool stage2, long long wave, cudaStream_t st) {
+  const int parts = stage_parts(a.ncells, wave);
+  if (!shear) launch_stage_physics<EOS, false, false, MIXED>(a, stage2, parts, st);
+  else if (!bulk) launch_stage_physics<EOS, true, false, MIXED>(a, stage2, parts, st);
+  else launch_stage_physics<EOS, true, true, MIXED>(a, stage2, parts, st);
+  return cudaGetLastError();
+}
+
+template <int EOS, bool MIXED, bool SHEAR, bool BULK, bool STAGE2>
+cudaError_t prepare_stage_kernel() {
+  const size_t smem = stage_smem_bytes<SHEAR, BULK>();
+  cudaError_t e = allow_stage_smem(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, smem);
+  if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, smem);
+  return e;
+}
+
+template <int EOS, bool MIXED>
+cudaError_t prepare_stages_of() {
+  cudaError_t e = prepare_stage_kernel<EOS, MIXED, false, false, false>();
+  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, false, false, true>();
+  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, false, false>();
+  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, false, true>();
+  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, true, false>();
+  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, true, true>();
+  return e;
+}
+
+}  // namespace gvh

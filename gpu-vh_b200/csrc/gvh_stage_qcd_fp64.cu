@@ -1,0 +1,11 @@
+// gvh_stage_qcd_fp64.cu -- the stage kernels of the QCD equation of state, plain FP64.
+#include "gvh_stage_launch.cuh"
+
+namespace gvh {
+
+cudaError_t prepare_qcd_fp64() { return prepare_stages_of<EOS_QCD, false>(); }
+cudaError_t launch_qcd_fp64(const StageArgs &a, int shear, int bulk, bool stage2, long long wave, cudaStream_t st) {
+  return launch_stage_of<EOS_QCD, false>(a, shear, bulk, stage2, wave, st);
+}
+
+}  // namespace gvh

@@ -21,9 +21,11 @@ NVCC_FLAGS = [
 
 
 def sources() -> list[str]:
-    return [os.path.join(CSRC, "gvh_capi.cu"), os.path.join(CSRC, "gvh_batch.cu"), os.path.join(CSRC, "gvh_plugin.cpp"),
-            os.path.join(CSRC, "gvh_noalloc.cu"), os.path.join(CSRC, "gvh_surface.cu"),
-            os.path.join(CSRC, "gvh_surface_host.cpp"), os.path.join(CSRC, "gvh_surface_rows.cu")]
+    # the slowest to compile first
+    names = ["gvh_batch.cu", "gvh_stage_qcd_fp64.cu", "gvh_stage_qcd_mixed.cu", "gvh_stage_conformal_fp64.cu",
+             "gvh_stage_conformal_mixed.cu", "gvh_surface_rows.cu", "gvh_surface.cu", "gvh_capi.cu", "gvh_noalloc.cu",
+             "gvh_plugin.cpp", "gvh_surface_host.cpp"]
+    return [os.path.join(CSRC, n) for n in names]
 
 
 # per-file flags: the device surface rows repeat the host's arithmetic operation for operation
