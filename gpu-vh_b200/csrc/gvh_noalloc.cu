@@ -48,6 +48,7 @@ __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
 
 std::mutex g_setup_mutex;
 std::atomic<unsigned char *> g_scratch_ptr[kMaxDevices];
+long long g_wave_cells[kMaxDevices];  // written before g_scratch_ptr is published
 
 thread_local std::string g_noalloc_error;
 
@@ -76,6 +77,10 @@ int scratch_address(int dev, unsigned char **out) {
       err = prepare_stage_kernels();
       if (err != cudaSuccess)
         return nfail(GVH_ERR_CUDA, "stage kernel set-up on device %d: %s", dev, cudaGetErrorString(err));
+      int sms = 0;
+      err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      if (err != cudaSuccess) return nfail(GVH_ERR_CUDA, "SM count of device %d: %s", dev, cudaGetErrorString(err));
+      g_wave_cells[dev] = stage_wave_cells(sms);
       g_scratch_ptr[dev].store(p, std::memory_order_release);
     }
   }
@@ -179,8 +184,8 @@ int gvh_rk2_step_noalloc(const gvh_lattice_params *L, const gvh_hydro_params *H,
   a2.qin = qS; a2.qn = q; a2.qout = q;
   a2.pin = pS; a2.pout = p;
   a2.uin = uS; a2.uprev = u; a2.uout = u_next;
-  err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a1, false, 0, st);
-  if (err == cudaSuccess) err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a2, true, 0, st);
+  err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a1, false, g_wave_cells[dev], st);
+  if (err == cudaSuccess) err = launch_stage(o.eos, o.shear, o.bulk, o.precision, a2, true, g_wave_cells[dev], st);
   if (err != cudaSuccess) return nfail(GVH_ERR_CUDA, "stage launch: %s", cudaGetErrorString(err));
   if (status_out) {
     err = cudaMemcpyAsync(status_out, status, sizeof(unsigned), cudaMemcpyDeviceToHost, st);

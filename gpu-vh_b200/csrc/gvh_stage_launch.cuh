@@ -8,15 +8,26 @@
 namespace gvh {
 
 // A lattice smaller than one wave of the one-thread-per-cell kernel (75,776 cells on 148 SMs) takes
-// four threads per cell: 33x33x17 conformal 49.9 -> 28.7 us per step, 61x61x1 QCD 56.3 -> 32.8;
-// a lattice that fills the GPU loses by it (131x131x61: 1.44 -> 2.14 ms).
-inline int stage_parts(long long ncells, long long wave) { return ncells < wave ? 4 : 1; }
+// the kernel whose waves it fills best: a wave of PARTS threads per cell holds 1/PARTS of the
+// cells and takes about 0.033 ms per step (PARTS = 4), 0.056 (2), 0.097 (1) for QCD with shear
+// and bulk, FP64. Measured, ms per step with 4 / 2 / 1: 18,513 cells 0.034 / 0.042 / 0.057;
+// 35,301 cells 0.063 / 0.055 / 0.066; 46,575 cells 0.087 / 0.089 / 0.092; 59,823 cells
+// 0.121 / 0.105 / 0.101; 81,608 cells 0.150 / 0.136 / 0.130. Mixed and conformal order alike.
+inline int stage_parts(long long ncells, long long wave) {
+  if (4 * ncells <= wave) return 4;
+  if (2 * ncells <= wave) return 2;
+  if (4 * ncells <= 3 * wave) return 4;
+  return 1;
+}
 
 template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
 void launch_stage_kernel(const StageArgs &a, int parts, cudaStream_t st) {
   const size_t smem = stage_smem_bytes<SHEAR, BULK>();
   if (parts == 4)
     launch_overlapped(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, split_grid(a.ncells, 4), kBlock, smem,
+                      st, a);
+  else if (parts == 2)
+    launch_overlapped(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 2>, split_grid(a.ncells, 2), kBlock, smem,
                       st, a);
   else
     launch_overlapped(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, stage_grid(a.ncells), kBlock, smem, st, a);
@@ -41,6 +52,7 @@ template <int EOS, bool MIXED, bool SHEAR, bool BULK, bool STAGE2>
 cudaError_t prepare_stage_kernel() {
   const size_t smem = stage_smem_bytes<SHEAR, BULK>();
   cudaError_t e = allow_stage_smem(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, smem);
+  if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 2>, smem);
   if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, smem);
   return e;
 }

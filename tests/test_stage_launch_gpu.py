@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import gvh
-from helpers import rich_state
+from helpers import rel_err, rich_state
 from test_zz_no_alloc import bound, stack
 
 pytestmark = pytest.mark.gpu
@@ -88,3 +88,57 @@ def test_captured_allocation_free_step():
     torch.cuda.synchronize()
     for a, b in zip(state + [nxt], want):
         assert torch.equal(a, b)
+
+
+# The kernels a lattice smaller than one wave takes (eight warps per 32 cells, four or two threads
+# per cell, one thread per cell), on both sides of each rule's line for 148 SMs: 9,472, 18,944,
+# 37,888 and 56,832 cells; with a partial last block, one-cell axes, and sizes of a few cells.
+PART_SHAPES = [(1, 1, 1), (3, 1, 1), (1, 5, 7), (37, 32, 8), (37, 32, 9), (37, 32, 16), (37, 32, 17), (37, 64, 16),
+               (37, 64, 17), (37, 96, 16), (37, 96, 17), (97, 97, 1), (101, 101, 1)]
+
+
+@pytest.mark.parametrize("physics", ["qcd_bulk", "conformal_shear", "qcd_ideal"])
+@pytest.mark.parametrize("shape", PART_SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_small_lattice_kernels_match_the_oracle(shape, physics):
+    """One step against the oracle on both sides of every line of the rule. Tolerance as the
+    parity tests': 1e-12 of the field's maximum, 1e-9 with the QCD solver."""
+    import oracle
+
+    opts = {"qcd_bulk": dict(conformal=False, shear=True, bulk=True, theta=2.0),
+            "conformal_shear": dict(conformal=True, shear=True, bulk=False, theta=1.8),
+            "qcd_ideal": dict(conformal=False, shear=False, bulk=False, theta=2.0)}[physics]
+    nx, ny, nz = shape
+    kw = dict(nx=nx, ny=ny, nz=nz, dx=0.3, dy=0.3, dz=0.3, dt=0.01, etabar=0.16, **opts)
+    G, O = gvh.Lattice(**kw), oracle.OracleLattice(**kw)
+    prim = rich_state(G, seed=13, spacing=6.0 / max(nx, ny))
+    G.set_primitive(prim)
+    O.set_primitive(prim)
+    G.step(0.5, 0.01)
+    O.step(0.5, 0.01)
+    assert G.status() == 0
+    sg, so = G.get_state(), O.get_state()
+    for k in G.field_names:
+        assert rel_err(G.interior(sg[k]), O.interior(so[k])) <= (1e-12 if opts["conformal"] else 1e-9), k
+    tol = 1e-12 if opts["conformal"] else 1e-9
+    a, b = G.max_propagation_speed(), O.max_propagation_speed()
+    assert abs(a - b) <= tol * max(b, 1e-30)
+
+
+@pytest.mark.parametrize("shape", [(21, 19, 17), (37, 32, 16), (37, 64, 16), (97, 90, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_mixed_small_lattice_kernels_match_a_batch(shape):
+    """The mixed path on the small-lattice kernels against a batch's one-thread-per-cell kernel, three
+    steps. The mixed path's bar (test_zz_no_alloc): the same FP32 expressions, whose multiply-add
+    contraction may differ between kernels."""
+    nx, ny, nz = shape
+    L = gvh.Lattice(nx, ny, nz, 0.3, 0.3, 0.3, 0.01, 0.16, precision="mixed", tau0=0.5)
+    prim = rich_state(L, seed=5, spacing=6.0 / max(nx, ny))
+    L.set_primitive(prim)
+    B = gvh.Batch(64 << 20, precision="mixed")
+    eid = B.add_event(nx, ny, nz, 0.3, 0.3, 0.3, 0.01, 0.16, prim, tau0=0.5)
+    for n in range(3):
+        L.step(0.5 + n * 0.01, 0.01)
+    B.step(3)
+    a, b = L.get_state(), B.get_state(eid)
+    for k in L.field_names:
+        assert rel_err(L.interior(a[k]), L.interior(b[k])) <= 1e-6, k
