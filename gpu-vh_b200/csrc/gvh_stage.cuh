@@ -182,7 +182,7 @@ __device__ __forceinline__ FaceSpeeds<double> face_speeds(const StageArgs &a, in
   }
   if (__builtin_expect(bad, 0)) {
     double v[4];
-    status |= face_velocities_general<EOS, NR>(a.t_euler, axis, cache, kBlock, g0.e, v);
+    status |= face_velocities_general<EOS, NR, 4>(a.t_euler, axis, cache, kBlock, g0.e, v);
     w[0] = v[0]; w[1] = v[1]; w[2] = v[2]; w[3] = v[3];
   }
   FaceSpeeds<double> f;
@@ -441,7 +441,8 @@ __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, in
 
 // The rest of a stage for one cell once out holds its Euler update: the Heun combination
 // (stage 2), primitive recovery at the new time, regulation, and the writes. Returns e.
-template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED, int OSTRIDE>
+// COMBINED: out already holds the combination.
+template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED, int OSTRIDE, bool COMBINED = false>
 __device__ __forceinline__ double stage_finish(const StageArgs &a, long long s, const double *out, const GuessEos &g0,
                                                unsigned status) {
   constexpr int NQ = NComp<SHEAR, BULK>::value;
@@ -449,7 +450,7 @@ __device__ __forceinline__ double stage_finish(const StageArgs &a, long long s, 
   double o[NQ];
 #pragma unroll
   for (int n = 0; n < NQ; ++n) o[n] = out[n * OSTRIDE];
-  if (STAGE2) {
+  if (STAGE2 && !COMBINED) {
 #pragma unroll
     for (int n = 0; n < NQ; ++n) o[n] = (o[n] + a.qn[n * a.cs + s]) * 0.5;
   }
@@ -746,6 +747,183 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
     if ((threadIdx.x & 31) == 0) atomicMax(a.speed_max, b);
+  }
+}
+
+// ---- the smallest lattices: one cell's stage on eight warps ------------------------------
+// Below an eighth of a wave (9,472 cells on 148 SMs) even PARTS = 4 leaves most SMs empty, and
+// an axis is the longest chain of a stage: its four recoveries and twice fifteen fluxes. Here
+// a block of eight warps takes 32 cells: warp 0 their source terms, warps 1..6 one face of one
+// axis each (two recoveries, fifteen fluxes), warp 7 the axes' pi, Pi derivative sources. After a
+// barrier the eight warps share the components of the Euler update (and the Heun combination),
+// then warp 0 finishes the cells. The expressions of kt_stage_kernel's mixed path bit for bit, of
+// its FP64 path to rounding.
+constexpr int kFaceBlock = 256;
+constexpr int kFaceCells = 32;
+
+inline dim3 faces_grid(long long ncells) { return dim3((unsigned)((ncells + kFaceCells - 1) / kFaceCells)); }
+
+// Per thread: NQ face fluxes (or updates, or sources) and two half-cell states per root-find
+// component.
+template <bool SHEAR, bool BULK>
+constexpr size_t faces_smem_bytes() {
+  return (size_t)(NComp<SHEAR, BULK>::value + 2 * (4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0))) * kFaceBlock * sizeof(double);
+}
+
+// The doubled KT flux H of every component through one face of the axis, flux[n * kFaceBlock]
+// (face_speeds and axis_update for one of the two faces): o, the offsets of the four cells around
+// the face, the second and third beside it. Returns the face's propagation speed.
+template <int EOS, bool SHEAR, bool BULK, bool MIXED>
+__device__ __forceinline__ double face_flux(const StageArgs &a, int s, int axis, const int (&o)[4], const GuessEos &g0,
+                                            double *flux, double *cache, unsigned &status) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  constexpr int NQ = NComp<SHEAR, BULK>::value;
+  constexpr int NR = 4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0);
+  constexpr int kPerPass = NR % 3 == 0 ? 3 : 4;
+  const double theta2 = 2 * a.theta;
+#pragma unroll kPerPass
+  for (int r = 0; r < NR; ++r) {
+    const double *q = a.qin + (size_t)(r < 8 ? r : 14) * a.cs + s;
+    const double q0 = ld_state(q + o[0]), q1 = ld_state(q + o[1]), q2 = ld_state(q + o[2]), q3 = ld_state(q + o[3]);
+    double D1, D2;
+    if (MIXED) {
+      const float t2f = (float)theta2;
+      const float d10 = (float)(q1 - q0), d21 = (float)(q2 - q1), d32 = (float)(q3 - q2);
+      D1 = slope2_from_differences(t2f, d10, (float)(q2 - q0), d21);
+      D2 = slope2_from_differences(t2f, d21, (float)(q3 - q1), d32);
+    } else {
+      D1 = limited_slope2(theta2, q0, q1, q2);
+      D2 = limited_slope2(theta2, q1, q2, q3);
+    }
+    cache[(2 * r) * kFaceBlock] = q2 - D2 * 0.25;      // right of the face
+    cache[(2 * r + 1) * kFaceBlock] = q1 + D1 * 0.25;  // left of it
+  }
+  double st[9][2], w[2];
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    st[r][0] = r < NR ? cache[(2 * r) * kFaceBlock] : 0.0;
+    st[r][1] = r < NR ? cache[(2 * r + 1) * kFaceBlock] : 0.0;
+  }
+  bool bad = false;
+  inferred_face_n<EOS, 2>(a.t_euler, axis, st[0], st[1], st[2], st[3], st[4], st[5], st[6], st[7], st[8], g0, w, bad);
+  if (__builtin_expect(bad, 0)) {
+    double v[2];
+    status |= face_velocities_general<EOS, NR, 2>(a.t_euler, axis, cache, kFaceBlock, g0.e, v);
+    w[0] = v[0]; w[1] = v[1];
+  }
+  const double speed = fmax(fabs(w[1]), fabs(w[0]));
+  const R wR = (R)w[0], wL = (R)w[1], as = (R)speed;
+  auto kt = [&](R fR, R fL) { return mul_rn(fR, wR) + mul_rn(fL, wL) - as * (fR - fL); };
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+    flux[(r < 8 ? r : NQ - 1) * kFaceBlock] =
+        (double)kt((R)cache[(2 * r) * kFaceBlock], (R)cache[(2 * r + 1) * kFaceBlock]);
+  if (SHEAR) {
+    const R th2 = R(2) * (R)a.theta;
+#pragma unroll 3
+    for (int n = 8; n < 14; ++n) {
+      const double *q = a.qin + (size_t)n * a.cs + s;
+      const R q0 = (R)ld_state(q + o[0]), q1 = (R)ld_state(q + o[1]);
+      const R q2 = (R)ld_state(q + o[2]), q3 = (R)ld_state(q + o[3]);
+      const R qu = R(0.25);
+      flux[n * kFaceBlock] = (double)kt(q2 - limited_slope2(th2, q1, q2, q3) * qu, q1 + limited_slope2(th2, q0, q1, q2) * qu);
+    }
+  }
+  return speed;
+}
+
+template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
+__global__ void __launch_bounds__(kFaceBlock, 2) kt_stage_faces_kernel(const StageArgs a) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  constexpr int NQ = NComp<SHEAR, BULK>::value;
+  const int lane = threadIdx.x % kFaceCells;
+  const int part = threadIdx.x / kFaceCells;
+  const long long id = (long long)blockIdx.x * kFaceCells + lane;
+  extern __shared__ double gvh_stage_smem[];
+  double *out = gvh_stage_smem + threadIdx.x;
+  double *cache = gvh_stage_smem + NQ * kFaceBlock + threadIdx.x;
+  eos_table_load<EOS>();
+  griddep_begin();
+  double speed = 0.0;
+  bool live = id < a.ncells;
+  int i = 0, j = 0, k = 0;
+  long long s = 0;
+  if (live) {
+    i = (int)(id % a.nx);
+    j = (int)((id / a.nx) % a.ny);
+    k = (int)(id / ((long long)a.nx * a.ny));
+    s = i + a.sy * j + a.sz * k;
+#ifdef GVH_BOUNDS_CHECK
+    if (!cell_stencil_ok(a, i, j, k)) {
+      if (part == 0) atomicOr(a.status, STATUS_BOUNDS);
+      live = false;
+    }
+#endif
+  }
+  auto offset = [&](int axis, int d) {  // of the (clamped) neighbour d cells along the axis
+    const int idx = axis == 0 ? i : axis == 1 ? j : k;
+    const int n = axis == 0 ? a.nx : axis == 1 ? a.ny : a.nz;
+    const int stride = axis == 0 ? 1 : axis == 1 ? (int)a.sy : (int)a.sz;
+    return (min(max(idx + d, 0), n - 1) - idx) * stride;
+  };
+  unsigned status = 0;
+  double ePrev = 0.0;
+  if (live) {
+    ePrev = a.e[s];
+    double uc[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) uc[m] = ld_state(a.uin + m * a.cs + s);
+    if (part == 0) {
+      stage_source<EOS, SHEAR, BULK, MIXED, kFaceBlock>(a, s, i, j, k, ePrev, uc, guess_eos<EOS>(ePrev), out);
+    } else if (part < 7) {
+      const int axis = (part - 1) >> 1, first = (part - 1) & 1 ? -2 : -1;  // face i+1/2, then i-1/2
+      const int n_axis = axis == 0 ? a.nx : axis == 1 ? a.ny : a.nz;
+      if (MIXED || n_axis > 1) {  // one-cell axes as in kt_stage_kernel
+        const int o[4] = {offset(axis, first), offset(axis, first + 1), offset(axis, first + 2), offset(axis, first + 3)};
+        const double as = face_flux<EOS, SHEAR, BULK, MIXED>(a, (int)s, axis, o, guess_eos<EOS>(ePrev), out, cache, status);
+        speed = n_axis > 1 ? as * (axis == 0 ? a.inv_dx : axis == 1 ? a.inv_dy : a.inv_dz) : 0.0;
+        if (status) atomicOr(a.status, status);
+      }
+    } else if (SHEAR) {
+#pragma unroll 1
+      for (int axis = 0; axis < 3; ++axis) {
+        const int o[5] = {0, offset(axis, -1), 0, offset(axis, 1), 0};
+        R Sa[4];
+        axis_pi_sources<SHEAR, BULK, R>(a, (int)s, axis, o, R(axis == 0 ? a.inv_dx : axis == 1 ? a.inv_dy : a.inv_dz),
+                                        uc, Sa);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) out[(4 * axis + m) * kFaceBlock] = (double)Sa[m];
+      }
+    }
+  }
+  __syncthreads();
+  if (live) {
+    double *cell = gvh_stage_smem + lane;  // part p's value of component n: cell[n * kFaceBlock + 32 p]
+    for (int n = part; n < NQ; n += 8) {
+      double *c = cell + n * kFaceBlock;
+      double o = c[0];
+#pragma unroll
+      for (int axis = 0; axis < 3; ++axis) {
+        const int n_axis = axis == 0 ? a.nx : axis == 1 ? a.ny : a.nz;
+        if (!MIXED && n_axis == 1) continue;
+        const R half_inv_d = R(0.5) * R(axis == 0 ? a.inv_dx : axis == 1 ? a.inv_dy : a.inv_dz);
+        R r = -(R)c[(1 + 2 * axis) * kFaceCells] + (R)c[(2 + 2 * axis) * kFaceCells];
+        r = r * half_inv_d;
+        if (SHEAR && n < 4) r += (R)cell[(4 * axis + n) * kFaceBlock + 7 * kFaceCells];
+        o += (double)r * a.dt;
+      }
+      if (STAGE2) o = (o + a.qn[n * a.cs + s]) * 0.5;
+      c[0] = o;
+    }
+  }
+  __syncthreads();
+  if (live && part == 0)
+    stage_finish<EOS, SHEAR, BULK, STAGE2, MIXED, kFaceBlock, true>(a, s, out, guess_eos<EOS>(ePrev), status);
+  if (!STAGE2 && a.speed_max) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(fmax(speed, 0.0));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if (lane == 0) atomicMax(a.speed_max, b);
   }
 }
 

@@ -12,8 +12,12 @@ namespace gvh {
 // cells and takes about 0.033 ms per step (PARTS = 4), 0.056 (2), 0.097 (1) for QCD with shear
 // and bulk, FP64. Measured, ms per step with 4 / 2 / 1: 18,513 cells 0.034 / 0.042 / 0.057;
 // 35,301 cells 0.063 / 0.055 / 0.066; 46,575 cells 0.087 / 0.089 / 0.092; 59,823 cells
-// 0.121 / 0.105 / 0.101; 81,608 cells 0.150 / 0.136 / 0.130. Mixed and conformal order alike.
+// 0.121 / 0.105 / 0.101; 81,608 cells 0.150 / 0.136 / 0.130. Eight warps per 32 cells
+// (kt_stage_faces_kernel) fill their wave with an eighth: 720 cells 0.0164 ms against 0.0238 with
+// PARTS = 4, 3,721 (2+1D) 0.0185 / 0.0260, 9,261 cells 0.0221 / 0.0284. Mixed and conformal order
+// alike.
 inline int stage_parts(long long ncells, long long wave) {
+  if (8 * ncells <= wave) return 8;
   if (4 * ncells <= wave) return 4;
   if (2 * ncells <= wave) return 2;
   if (4 * ncells <= 3 * wave) return 4;
@@ -23,7 +27,10 @@ inline int stage_parts(long long ncells, long long wave) {
 template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
 void launch_stage_kernel(const StageArgs &a, int parts, cudaStream_t st) {
   const size_t smem = stage_smem_bytes<SHEAR, BULK>();
-  if (parts == 4)
+  if (parts == 8)
+    launch_overlapped(kt_stage_faces_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, faces_grid(a.ncells), kFaceBlock,
+                      faces_smem_bytes<SHEAR, BULK>(), st, a);
+  else if (parts == 4)
     launch_overlapped(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, split_grid(a.ncells, 4), kBlock, smem,
                       st, a);
   else if (parts == 2)
@@ -54,6 +61,8 @@ cudaError_t prepare_stage_kernel() {
   cudaError_t e = allow_stage_smem(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, smem);
   if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 2>, smem);
   if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, smem);
+  if (e == cudaSuccess)
+    e = allow_stage_smem(kt_stage_faces_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, faces_smem_bytes<SHEAR, BULK>());
   return e;
 }
 
