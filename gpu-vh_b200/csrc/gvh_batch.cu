@@ -671,7 +671,7 @@ int admit_event(gvh_batch *b, const gvh_lattice_params *L, const gvh_hydro_param
     for (int m = 0; m < 4; ++m) dst.p[1 + m] = u[0] + m * h.cs;
     for (int n = 4; n < b->nq; ++n) dst.p[5 + n - 4] = qA + n * h.cs;
     Pack pk{h.nx, h.ny, h.nz, (long long)h.nx, (long long)h.nx * h.ny, h.ng};
-    pack_kernel<<<blocks, 256, 0, b->stream>>>(pk, n_prim, b->staging, dst);
+    pack_kernel<<<layout_grid(h.ncells, n_prim), kLayoutBlock, 0, b->stream>>>(pk, n_prim, b->staging, dst);
   }
   if (b->opts.eos == GVH_EOS_CONFORMAL)
     init_conserved_kernel<EOS_CONFORMAL><<<blocks, 256, 0, b->stream>>>(h.ncells, b->nq, h.cs, qA, e, pA, u[0], u[1], 0);
@@ -816,7 +816,7 @@ int gvh_batch_get_state(gvh_batch *b, int id, double *const *fields, int n_field
   for (int m = 0; m < 4; ++m) src.p[b->nq + 2 + m] = fields[b->nq + 2 + m] ? E.u[E.ucur] + m * h.cs : nullptr;
   for (int m = 0; m < 4; ++m) src.p[b->nq + 6 + m] = fields[b->nq + 6 + m] ? E.u[E.uprev] + m * h.cs : nullptr;
   Pack pk{h.nx, h.ny, h.nz, (long long)h.nx, (long long)h.nx * h.ny, h.ng};
-  unpack_kernel<<<(unsigned)((h.ng + 255) / 256), 256, 0, b->stream>>>(pk, n_fields, src, b->staging);
+  unpack_kernel<<<layout_grid(h.ng, n_fields), kLayoutBlock, 0, b->stream>>>(pk, n_fields, src, b->staging);
   BCUDA(cudaGetLastError());
   const size_t fb = h.ng * sizeof(double);
   for (int f = 0; f < n_fields; ++f)

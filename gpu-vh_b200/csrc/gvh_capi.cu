@@ -308,7 +308,7 @@ int gvh_set_state(gvh_handle *h, const double *const *fields, int n_fields) {
   }
   FieldTable dst = {};
   internal_fields(h, dst.p);
-  pack_kernel<<<(unsigned)((h->ncells + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_fields, h->staging, dst);
+  pack_kernel<<<layout_grid(h->ncells, n_fields), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_fields, h->staging, dst);
   GVH_CUDA(cudaGetLastError());
   GVH_CUDA(cudaStreamSynchronize(h->stream));  // the caller may reuse its arrays on return
   return GVH_OK;
@@ -323,7 +323,7 @@ int gvh_get_state(gvh_handle *h, double *const *fields, int n_fields) {
   internal_fields(h, src.p);
   for (int f = 0; f < n_fields; ++f)
     if (!fields[f]) src.p[f] = nullptr;
-  unpack_kernel<<<(unsigned)((h->ng + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_fields, src, h->staging);
+  unpack_kernel<<<layout_grid(h->ng, n_fields), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_fields, src, h->staging);
   GVH_CUDA(cudaGetLastError());
   const size_t fb = h->ng * sizeof(double);
   for (int f = 0; f < n_fields; ++f)
@@ -349,9 +349,8 @@ int gvh_gather_state_device(gvh_handle *h, const void *const *fields, int n_fiel
   if ((rc = set_device(h))) return rc;
   FieldTable dst = {};
   internal_fields(h, dst.p);
-  const unsigned blocks = (unsigned)((h->ncells + 255) / 256);
-  if (elem_bytes == 4) gather_ref_kernel<float><<<blocks, 256, 0, h->stream>>>(make_pack(h), n_fields, src, dst);
-  else gather_ref_kernel<double><<<blocks, 256, 0, h->stream>>>(make_pack(h), n_fields, src, dst);
+  launch_overlapped(elem_bytes == 4 ? gather_ref_kernel<float> : gather_ref_kernel<double>,
+                    layout_grid(h->ncells, n_fields), kLayoutBlock, 0, h->stream, make_pack(h), n_fields, src, dst);
   GVH_CUDA(cudaGetLastError());
   return GVH_OK;
 }
@@ -368,9 +367,8 @@ int gvh_scatter_state_device(gvh_handle *h, void *const *fields, int n_fields, i
   for (int f = 0; f < n_fields; ++f) dst.p[f] = fields[f];
   FieldTable src = {};
   internal_fields(h, src.p);
-  const unsigned blocks = (unsigned)((h->ng + 255) / 256);
-  if (elem_bytes == 4) scatter_ref_kernel<float><<<blocks, 256, 0, h->stream>>>(make_pack(h), n_fields, src, dst);
-  else scatter_ref_kernel<double><<<blocks, 256, 0, h->stream>>>(make_pack(h), n_fields, src, dst);
+  launch_overlapped(elem_bytes == 4 ? scatter_ref_kernel<float> : scatter_ref_kernel<double>,
+                    layout_grid(h->ng, n_fields), kLayoutBlock, 0, h->stream, make_pack(h), n_fields, src, dst);
   GVH_CUDA(cudaGetLastError());
   return GVH_OK;
 }
@@ -394,7 +392,7 @@ int gvh_set_primitive_state_p(gvh_handle *h, const double *const *prim, int n_pr
   for (int n = 4; n < h->nq; ++n) dst.p[5 + n - 4] = h->qA + n * h->cs;
   dst.p[n_prim] = h->pA;
   const int n_pack = n_prim + (p_ghosted ? 1 : 0);
-  pack_kernel<<<(unsigned)((h->ncells + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_pack, h->staging, dst);
+  pack_kernel<<<layout_grid(h->ncells, n_pack), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_pack, h->staging, dst);
   GVH_CUDA(cudaGetLastError());
   const unsigned blocks = (unsigned)((h->ncells + 255) / 256);
   if (h->eos == GVH_EOS_CONFORMAL)
@@ -513,7 +511,7 @@ int gvh_get_validity(gvh_handle *h, double *const *fields, int n_fields) {
   if ((rc = set_device(h)) || (rc = ensure_staging(h))) return rc;
   FieldTable src = {};
   for (int f = 0; f < kValidityFields; ++f) src.p[f] = fields[f] ? h->diag + (size_t)f * h->cs : nullptr;
-  unpack_kernel<<<(unsigned)((h->ng + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_fields, src, h->staging);
+  unpack_kernel<<<layout_grid(h->ng, n_fields), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_fields, src, h->staging);
   GVH_CUDA(cudaGetLastError());
   const size_t fb = h->ng * sizeof(double);
   for (int f = 0; f < n_fields; ++f)
@@ -705,7 +703,7 @@ int gvh_set_state_async(gvh_handle *h, const double *const *fields, int n_fields
   }
   GVH_CUDA(cudaEventRecord(h->ev_in_ready, h->s_h2d));
   GVH_CUDA(cudaStreamWaitEvent(h->stream, h->ev_in_ready, 0));
-  pack_kernel<<<(unsigned)((h->ncells + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_fields, staging, dst);
+  pack_kernel<<<layout_grid(h->ncells, n_fields), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_fields, staging, dst);
   GVH_CUDA(cudaGetLastError());
   GVH_CUDA(cudaEventRecord(h->ev_in_free[slot], h->stream));
   h->in_slot = slot ^ 1;
@@ -726,7 +724,7 @@ int gvh_get_state_async(gvh_handle *h, double *const *fields, int n_fields) {
   const int slot = h->out_slot;
   double *const staging = h->staging_out[slot];
   GVH_CUDA(cudaStreamWaitEvent(h->stream, h->ev_out_free[slot], 0));
-  unpack_kernel<<<(unsigned)((h->ng + 255) / 256), 256, 0, h->stream>>>(make_pack(h), n_fields, src, staging);
+  unpack_kernel<<<layout_grid(h->ng, n_fields), kLayoutBlock, 0, h->stream>>>(make_pack(h), n_fields, src, staging);
   GVH_CUDA(cudaGetLastError());
   GVH_CUDA(cudaEventRecord(h->ev_out_ready, h->stream));
   GVH_CUDA(cudaStreamWaitEvent(h->s_d2h, h->ev_out_ready, 0));

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/gvh.h"
+#include "gvh_launch.cuh"
 #include "gvh_physics.cuh"
 
 namespace {
@@ -28,29 +29,16 @@ struct FieldTable {
   double *p[32];
 };
 
-// staging (nf fields, ghosted) -> internal fields dst.p[f] (interior); null entries are skipped
-__global__ void pack_kernel(Pack p, int nf, const double *__restrict__ staging, FieldTable dst) {
-  long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long n = (long long)p.nx * p.ny * p.nz;
-  if (id >= n) return;
-  int i = id % p.nx, j = (id / p.nx) % p.ny, k = id / ((long long)p.nx * p.ny);
-  long long r = ref_index(p, i, j, k), s = i + p.sy * j + p.sz * k;
-  for (int f = 0; f < nf; ++f)
-    if (dst.p[f]) dst.p[f][s] = staging[f * p.ng + r];
-}
-
-// internal fields src.p[f] -> staging (ghosted, every ghost cell filled from the nearest
-// interior cell: the reference's zero-gradient faces, edges and corners alike); null entries
-// are skipped
-__global__ void unpack_kernel(Pack p, int nf, FieldTable src, double *__restrict__ staging) {
-  long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long n = p.ng;
-  if (id >= n) return;
-  int gi = id % (p.nx + 4), gj = (id / (p.nx + 4)) % (p.ny + 4), gk = id / ((long long)(p.nx + 4) * (p.ny + 4));
-  int i = min(max(gi - 2, 0), p.nx - 1), j = min(max(gj - 2, 0), p.ny - 1), k = min(max(gk - 2, 0), p.nz - 1);
-  long long s = i + p.sy * j + p.sz * k;
-  for (int f = 0; f < nf; ++f)
-    if (src.p[f]) staging[f * p.ng + id] = src.p[f][s];
+// The conversions move nf fields of one cell. A thread takes up to kFieldsPerThread of them, all
+// its loads before its stores, and blockIdx.y takes the next ones (layout_grid): one thread walking
+// through the 25 fields waits for each load before it issues the next. Bound by that latency on
+// small lattices and by HBM on large ones: gather / scatter of 12x10x6 8.3 / 8.4 -> 5.3 / 5.1 us,
+// 101x101x31 39 / 40 -> 19 / 24, 131x131x61 88 / 93 -> 69 / 74 (0.45 GB, 68 us at 6.55 TB/s).
+constexpr int kLayoutBlock = 256;
+constexpr int kFieldsPerThread = 8;
+inline dim3 layout_grid(long long cells, int nf) {
+  return dim3((unsigned)((cells + kLayoutBlock - 1) / kLayoutBlock),
+              (unsigned)((nf + kFieldsPerThread - 1) / kFieldsPerThread));
 }
 
 // Arrays in the element type of the caller (the reference's PRECISION: float as shipped,
@@ -59,32 +47,79 @@ struct RefTable {
   void *p[32];
 };
 
-// The reference's ghosted device arrays (type T) -> internal fields dst.p[f] (interior),
-// converted to double; one launch for every field. Null entries on either side are skipped.
-template <class T>
-__global__ void gather_ref_kernel(Pack p, int nf, RefTable src, FieldTable dst) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n = (long long)p.nx * p.ny * p.nz;
-  if (id >= n) return;
-  const int i = id % p.nx, j = (id / p.nx) % p.ny, k = id / ((long long)p.nx * p.ny);
-  const long long r = ref_index(p, i, j, k), s = i + p.sy * j + p.sz * k;
-  for (int f = 0; f < nf; ++f)
-    if (dst.p[f] && src.p[f]) dst.p[f][s] = (double)static_cast<const T *>(src.p[f])[r];
+// The fields f0.. of one cell: to(f) = from(f) where both are given (null entries are skipped).
+template <class From, class To, class Load, class Store>
+__device__ __forceinline__ void move_fields(int nf, From from, To to, Load load, Store store) {
+  const int f0 = blockIdx.y * kFieldsPerThread;
+  double v[kFieldsPerThread];
+#pragma unroll
+  for (int m = 0; m < kFieldsPerThread; ++m)
+    v[m] = f0 + m < nf && to(f0 + m) && from(f0 + m) ? load(f0 + m) : 0.0;
+#pragma unroll
+  for (int m = 0; m < kFieldsPerThread; ++m)
+    if (f0 + m < nf && to(f0 + m) && from(f0 + m)) store(f0 + m, v[m]);
 }
 
-// Internal fields src.p[f] -> the reference's ghosted device arrays (type T), every ghost
-// cell filled from the nearest interior cell (GhostCells.cu:15-144 fills the faces; edges and
-// corners get the same clamped value); null entries are skipped.
-template <class T>
-__global__ void scatter_ref_kernel(Pack p, int nf, FieldTable src, RefTable dst) {
+// Interior cell of a thread: its index s in the internal layout and r in the ghosted one.
+__device__ __forceinline__ bool interior_cell(const Pack &p, long long &s, long long &r) {
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= p.ng) return;
+  if (id >= (long long)p.nx * p.ny * p.nz) return false;
+  const int i = id % p.nx, j = (id / p.nx) % p.ny, k = id / ((long long)p.nx * p.ny);
+  r = ref_index(p, i, j, k);
+  s = i + p.sy * j + p.sz * k;
+  return true;
+}
+
+// Ghosted cell of a thread, id, and the nearest interior cell s (the reference's zero-gradient
+// faces, GhostCells.cu:15-144; edges and corners get the same clamped value).
+__device__ __forceinline__ bool ghosted_cell(const Pack &p, long long &id, long long &s) {
+  id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= p.ng) return false;
   const int gi = id % (p.nx + 4), gj = (id / (p.nx + 4)) % (p.ny + 4);
   const int gk = id / ((long long)(p.nx + 4) * (p.ny + 4));
   const int i = min(max(gi - 2, 0), p.nx - 1), j = min(max(gj - 2, 0), p.ny - 1), k = min(max(gk - 2, 0), p.nz - 1);
-  const long long s = i + p.sy * j + p.sz * k;
-  for (int f = 0; f < nf; ++f)
-    if (dst.p[f] && src.p[f]) static_cast<T *>(dst.p[f])[id] = (T)src.p[f][s];
+  s = i + p.sy * j + p.sz * k;
+  return true;
+}
+
+// staging (nf fields, ghosted) -> internal fields dst.p[f] (interior); null entries are skipped
+__global__ void pack_kernel(Pack p, int nf, const double *__restrict__ staging, FieldTable dst) {
+  long long s, r;
+  if (!interior_cell(p, s, r)) return;
+  move_fields(nf, [](int) { return true; }, [&](int f) { return dst.p[f] != nullptr; },
+              [&](int f) { return staging[f * p.ng + r]; }, [&](int f, double v) { dst.p[f][s] = v; });
+}
+
+// internal fields src.p[f] -> staging (ghosted); null entries are skipped
+__global__ void unpack_kernel(Pack p, int nf, FieldTable src, double *__restrict__ staging) {
+  long long id, s;
+  if (!ghosted_cell(p, id, s)) return;
+  move_fields(nf, [&](int f) { return src.p[f] != nullptr; }, [](int) { return true; },
+              [&](int f) { return src.p[f][s]; }, [&](int f, double v) { staging[f * p.ng + id] = v; });
+}
+
+// The reference's ghosted device arrays (type T) -> internal fields dst.p[f] (interior),
+// converted to double; one launch for every field. Null entries on either side are skipped.
+// Launched overlapped, like the stages between it and scatter_ref_kernel.
+template <class T>
+__global__ void gather_ref_kernel(Pack p, int nf, RefTable src, FieldTable dst) {
+  griddep_begin();
+  long long s, r;
+  if (!interior_cell(p, s, r)) return;
+  move_fields(nf, [&](int f) { return src.p[f] != nullptr; }, [&](int f) { return dst.p[f] != nullptr; },
+              [&](int f) { return (double)static_cast<const T *>(src.p[f])[r]; },
+              [&](int f, double v) { dst.p[f][s] = v; });
+}
+
+// Internal fields src.p[f] -> the reference's ghosted device arrays (type T), every ghost
+// cell filled; null entries are skipped.
+template <class T>
+__global__ void scatter_ref_kernel(Pack p, int nf, FieldTable src, RefTable dst) {
+  griddep_begin();
+  long long id, s;
+  if (!ghosted_cell(p, id, s)) return;
+  move_fields(nf, [&](int f) { return src.p[f] != nullptr; }, [&](int f) { return dst.p[f] != nullptr; },
+              [&](int f) { return src.p[f][s]; }, [&](int f, double v) { static_cast<T *>(dst.p[f])[id] = (T)v; });
 }
 
 // T^{tau mu} from primitives (DynamicalVariables.cu:349-392 with EnergyMomentumTensor.cu

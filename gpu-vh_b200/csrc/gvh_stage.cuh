@@ -29,6 +29,7 @@
 
 #include <type_traits>
 
+#include "gvh_launch.cuh"
 #include "gvh_physics.cuh"
 #include "gvh_sources.cuh"
 
@@ -601,32 +602,6 @@ __device__ __forceinline__ double stage_cell(const StageArgs &a, long long id, d
   const int j = (int)((id / a.nx) % a.ny);
   const int k = (int)(id / ((long long)a.nx * a.ny));
   return stage_cell_ijk<EOS, SHEAR, BULK, STAGE2, MIXED>(a, i, j, k, speed);
-}
-
-// Consecutive stage launches overlap their edges (programmatic dependent launch): the next
-// kernel's blocks are set up while the last blocks of this one finish, and wait in
-// griddep_begin, before their first access to the state, until the kernel before has ended and
-// its writes are visible. Launched without the attribute both calls do nothing. A 12x10x6 step
-// takes 28.7 -> 22.6 us, 33x33x17 conformal 28.7 -> 24.6, 131x131x61 1.239 -> 1.236 ms.
-__device__ __forceinline__ void griddep_begin() {
-  cudaGridDependencySynchronize();
-  cudaTriggerProgrammaticLaunchCompletion();
-}
-// Launches a kernel that calls griddep_begin (errors are left for cudaGetLastError).
-template <class... Params, class... Args>
-inline void launch_overlapped(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream,
-                              Args... args) {
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 // The grid of a stage launch: one block per kBlock consecutive cells (interior index order).
