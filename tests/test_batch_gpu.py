@@ -274,3 +274,43 @@ def test_empty_batch_and_bad_ids():
     again = B.add_event(**kw, prim=prim, tau0=t0_ev)
     B.step(1)
     assert B.info(again).step == 1
+
+
+def test_admissions_and_retirements_between_captures():
+    """The step's graph follows admissions and retirements at the next step, also where that step
+    is itself captured into a caller's graph: the events end where they end alone."""
+    import torch
+
+    def event(B, seed, nx):
+        L = dict(nx=nx, ny=9, nz=4, dx=0.3, dy=0.3, dz=0.3, dt=0.01, etabar=0.16)
+        shape = gvh.Lattice(**L, conformal=False)
+        prim = rich_state(shape, seed=seed)
+        shape.close()
+        return B.add_event(**L, prim=prim, tau0=0.5)
+
+    def alone(seed, nx, steps):
+        B = gvh.Batch(16 << 20)
+        e = event(B, seed, nx)
+        B.step(steps)
+        s = B.get_state(e)
+        B.close()
+        return s
+
+    B = gvh.Batch(16 << 20)
+    stream = torch.cuda.Stream()
+    B.set_stream(stream.cuda_stream)
+    a, b = event(B, 1, 11), event(B, 2, 40)
+    B.step(2)
+    B.remove_event(a)
+    c = event(B, 3, 23)  # the tile count has changed: the next step's graph is stale
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        B.step(2)
+    g.replay()
+    torch.cuda.synchronize()
+    B.step(1)
+    for e, want in ((b, alone(2, 40, 5)), (c, alone(3, 23, 3))):
+        got = B.get_state(e)
+        for k, v in want.items():
+            np.testing.assert_array_equal(got[k], v, err_msg=k)
+    B.close()
