@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/gvh.h"
+#define GVH_BATCH_KERNELS  // bulk_zeta_over_s
 #include "gvh_layout.cuh"
 #include "gvh_nvtx.h"
 #include "gvh_stage.cuh"

@@ -17,7 +17,7 @@
 //
 // Per axis the flux is done in two phases to keep few values live: (A) the half-cell states
 // of the components the root find needs (T^{tau mu}, pi^{tau mu}, Pi) go to a shared-memory
-// cache, and the four face recoveries (one Newton solve at a time) give u^axis/u^tau on both
+// cache, and the four face recoveries (two Newton solves at a time) give u^axis/u^tau on both
 // sides of both faces; (B) the cached components, then pi^{ij} (5 loads, 3 limited slopes),
 // go through the two KT fluxes into the running update.
 //
@@ -120,7 +120,7 @@ __device__ __forceinline__ FaceSpeeds<double> face_speeds(const StageArgs &a, in
                                                        const GuessEos &g0, const PiSink &sink, double *cache,
                                                        unsigned &status) {
   // index f: 0 fwd R, 1 fwd L, 2 bwd R, 3 bwd L. The states go to the cache first; the four
-  // recoveries then read them back one at a time (runtime loops keep the code small:
+  // recoveries then read them back two at a time (runtime loops keep the code small:
   // instruction fetch, not arithmetic, is what the long straight-line variant waited on).
   constexpr int NR = 4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0);
   // three components per pass, or four where they divide without a rest: their 15 to 20 stencil
