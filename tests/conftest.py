@@ -28,3 +28,18 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_pyfunc_call(pyfuncitem):
+    """A test that needs a build of the reference's own sources (oracle/_ref, made where the
+    reference tree is present) skips where that build is absent."""
+    import oracle
+
+    try:
+        return (yield)
+    except FileNotFoundError as err:
+        path = str(err.args[0])
+        if not path.startswith(oracle.REF_DIR + os.sep):
+            raise
+        pytest.skip(f"reference build {os.path.basename(path)} not built (oracle/build_ref.py needs the reference tree)")
