@@ -10,16 +10,17 @@
 
 namespace gvh {
 
-// Division in the working precision: reciprocal-based in both, to rounding in FP64 (div_fast;
-// the divisors here -- tau, u^tau, eta/s, the fits' denominators, zeta/s -- are normal numbers
-// in any state that is not already lost, and a NaN or an infinity stays one or becomes NaN).
+// Division in the working precision: reciprocal-based in both, in FP64 within an ulp (div_fast). The
+// divisors here -- tau, u^tau, the fits' denominators, zeta/s -- are normal numbers far from 2^1021
+// in any state that is not already lost; where one is not, the quotient is NaN or 0 and no status
+// bit is raised for it here (the recovery that follows sees the NaN).
 __device__ __forceinline__ double dv(double a, double b) { return div_fast(a, b); }
 __device__ __forceinline__ float dv(float a, float b) { return __fdividef(a, b); }
 // Division by a caller's setting, which may be any value: an infinite eta/s is valid (T / eta/s = 0:
 // no relaxation). Every cell takes the same branch.
 __device__ __forceinline__ double dv_setting(double a, double b) {
   const unsigned x = (unsigned)__double2hiint(b) & 0x7ff00000u;
-  return x - 0x00100000u < 0x7fb00000u ? div_fast(a, b) : a / b;  // 2^-1022 <= |b| < 2^1022, or not
+  return x - 0x00100000u < 0x7fb00000u ? div_fast(a, b) : a / b;  // 2^-1022 <= |b| < 2^1021, or not
 }
 __device__ __forceinline__ float dv_setting(float a, float b) { return dv(a, b); }
 
