@@ -717,7 +717,7 @@ int admit_event(gvh_batch *b, const gvh_lattice_params *L, const gvh_hydro_param
   E.dx = L->latticeSpacingX; E.dy = L->latticeSpacingY; E.dz = L->latticeSpacingRapidity;
   E.dt = L->latticeSpacingProperTime;
   E.inv_dx = 1.0 / E.dx; E.inv_dy = 1.0 / E.dy; E.inv_dz = 1.0 / E.dz; E.inv_dt = 1.0 / E.dt;
-  E.etabar = H->shearViscosityToEntropyDensity;
+  E.etabar = stage_etabar(H->shearViscosityToEntropyDensity);
   E.theta = b->opts.theta;
   E.cartesian = b->opts.coordinates == GVH_COORDINATES_CARTESIAN;
   const double T_reg = H->regulationTemperatureGeV / kHbarc;

@@ -16,13 +16,6 @@ namespace gvh {
 // bit is raised for it here (the recovery that follows sees the NaN).
 __device__ __forceinline__ double dv(double a, double b) { return div_fast(a, b); }
 __device__ __forceinline__ float dv(float a, float b) { return __fdividef(a, b); }
-// Division by a caller's setting, which may be any value: an infinite eta/s is valid (T / eta/s = 0:
-// no relaxation). Every cell takes the same branch.
-__device__ __forceinline__ double dv_setting(double a, double b) {
-  const unsigned x = (unsigned)__double2hiint(b) & 0x7ff00000u;
-  return x - 0x00100000u < 0x7fb00000u ? div_fast(a, b) : a / b;  // 2^-1022 <= |b| < 2^1021, or not
-}
-__device__ __forceinline__ float dv_setting(float a, float b) { return dv(a, b); }
 
 // Flow state and limited first derivatives at a cell.
 template <class R>
@@ -50,7 +43,7 @@ __device__ __forceinline__ void pimunu_rhs(R *rhs, R t, R etabar, R e, R p, cons
   const R dxuy = f.dxuy, dyuy = f.dyuy, dnuy = f.dnuy, dxun = f.dxun, dyun = f.dyun, dnun = f.dnun;
 
   R T = temperature<EOS>(e);
-  R taupiInv = R(kF02) * dv_setting(T, etabar);
+  R taupiInv = R(kF02) * dv(T, etabar);
   R beta_pi = R(kF02) * (e + p);
 
   R ut2 = ut * ut, un2 = un * un, t2 = t * t, t3 = t * t2;

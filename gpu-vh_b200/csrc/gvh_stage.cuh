@@ -91,6 +91,10 @@ __host__ __device__ inline void set_inverse_spacings(StageArgs &a) {
   a.inv_dt = 1.0 / a.dt;
 }
 
+// eta/s as the kernels take it. Infinity (no relaxation: T / eta/s = 0) is a valid setting without a
+// reciprocal in div_fast; a quotient below 1e-300 makes the same sums.
+inline double stage_etabar(double etabar) { return etabar > 0x1p1000 ? 0x1p1000 : etabar; }
+
 template <bool SHEAR, bool BULK>
 struct NComp {
   static constexpr int value = 4 + (SHEAR ? 10 : 0) + (BULK ? 1 : 0);
