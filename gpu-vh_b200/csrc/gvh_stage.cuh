@@ -432,7 +432,8 @@ __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, in
   if (SHEAR) {
     ShearT<R> pi{q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13]};
     R rhs[11];
-    pimunu_rhs<EOS, BULK, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk, g0.cs2);
+    pimunu_rhs<EOS, BULK, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk,
+                              BULK && !MIXED ? guess_cs2<EOS>(g0) : 0.0);
 #pragma unroll
     for (int n = 4; n < NQ; ++n) S[n] = rhs[n - 4];
   }

@@ -1,7 +1,9 @@
 // Device check of the building blocks of the primitive recovery, run by test_recovery_gpu.py:
 //   quotient, root: div_fast and sqrt_fast against CUDA's division and square root (which are
 //     correctly rounded), in units in the last place, over their operands' ranges, and what they
-//     give outside them.
+//     give outside them;
+//   solver: energy_from_conserved_n on states whose Newton divisors leave the range of div_fast, and
+//     c_s^2 at every energy.
 // Prints one line per check and the number of failures.
 #include <math.h>
 #include <stdint.h>
@@ -26,6 +28,26 @@ __global__ void root(int n, const double *a, double *fast, double *ieee) {
   if (i >= n) return;
   fast[i] = sqrt_fast(a[i]);
   ieee[i] = sqrt(a[i]);
+}
+// state i: guess g[i], M0, M, Pi
+__global__ void solve(int n, const double *s, double *e, int *bad) {
+  eos_table_load<EOS_QCD>();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const GuessEos g = guess_eos<EOS_QCD>(s[4 * i]);
+  double m0[1] = {s[4 * i + 1]}, m[1] = {s[4 * i + 2]}, pi[1] = {s[4 * i + 3]}, r[1];
+  bool b = false;
+  energy_from_conserved_n<EOS_QCD, 1>(g, m0, m, pi, r, b);
+  e[i] = r[0];
+  bad[i] = b;
+}
+// c_s^2 of a cell, and with the IEEE division
+__global__ void guess(int n, const double *e, double *fast, double *ieee) {
+  eos_table_load<EOS_QCD>();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  fast[i] = guess_cs2<EOS_QCD>(guess_eos<EOS_QCD>(e[i]));
+  ieee[i] = sound_speed2<EOS_QCD>(e[i]);
 }
 
 template <class T>
@@ -145,6 +167,38 @@ int main() {
     ok = true;
     for (double x : r) ok = ok && isnan(x);
     check("NaN for the root of 0, a subnormal, a negative number, infinity or NaN", ok, 0);
+  }
+  // Solver. With a huge Pi, A = H = Pi and the solution is e = B / Pi, B = M0 (M0 + Pi) - M. Whatever
+  // the size of the divisors (about Pi^2), a solve is handed to the general form or right (to the
+  // stop test's 1e-3; the tolerance adds the Newton step after it).
+  {
+    std::vector<double> s, want;
+    for (double Pi = 1e100; Pi < 1.3e154; Pi *= 1.05)
+      for (double root : {0.3, 0.7}) {
+        const double M0 = 10;
+        s.insert(s.end(), {0.2, M0, M0 * (M0 + Pi) - root * Pi, Pi});
+        want.push_back(root);
+      }
+    s.insert(s.end(), {0.2, 10, 10 * (10 + 1.3e154), 1.3e154});  // the first divisor is 2^1022.9
+    want.push_back(0);
+    Dev<double> ds(s), e(want.size());
+    Dev<int> bad(want.size());
+    solve<<<(int)((want.size() + 127) / 128), 128>>>((int)want.size(), ds.p, e.p, bad.p);
+    const std::vector<double> ge = e.get();
+    const std::vector<int> gb = bad.get();
+    double wrong = 0;
+    for (size_t i = 0; i < want.size(); ++i) wrong += !gb[i] && !(fabs(ge[i] - want[i]) <= 2e-3 * want[i]);
+    check("solves with divisors of any size: wrong and not handed on", wrong == 0, wrong);
+  }
+  {
+    std::vector<double> e;
+    for (double x = 1e-7; x < 5e24; x *= 1.01) e.push_back(x);
+    Dev<double> de(e), fast(e.size()), ieee(e.size());
+    guess<<<(int)((e.size() + 127) / 128), 128>>>((int)e.size(), de.p, fast.p, ieee.p);
+    const std::vector<double> f = fast.get(), q = ieee.get();
+    double worst = 0;
+    for (size_t i = 0; i < e.size(); ++i) worst = fmax(worst, ulps(f[i], q[i]));
+    check("c_s^2 of the guess, ulp", worst <= 1, worst);
   }
   const cudaError_t err = cudaDeviceSynchronize();
   check(cudaGetErrorString(err), err == cudaSuccess, 0);

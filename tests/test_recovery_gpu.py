@@ -1,5 +1,5 @@
 """The building blocks of the primitive recovery on the device (recovery_check.cu, built here with
-nvcc): quotient and square root against the IEEE operations."""
+nvcc): quotient and square root against the IEEE operations, solves with divisors of any size."""
 import os
 import shutil
 import subprocess
