@@ -280,10 +280,12 @@ __device__ __forceinline__ void axis_pi_sources(const StageArgs &a, int s, int a
 
 // Returns the axis's local propagation speed, max(a(i+1/2), a(i-1/2)) (SpectralRadius.cu:17-30).
 // dt: the time step, or 1 where out collects increments before that factor (the split kernel).
-template <int EOS, bool SHEAR, bool BULK, bool MIXED>
+// HALVES (mixed path), half 0 or 1: the increments, which are floats, are stored in that half of
+// out's elements; half < 0: added as without it.
+template <int EOS, bool SHEAR, bool BULK, bool MIXED, bool HALVES = false>
 __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axis, int idx, int n_axis, int stride,
                                               double inv_spacing, double dt, const GuessEos &g0, const double *uc,
-                                              double *out, double *cache, unsigned &status) {
+                                              double *out, double *cache, unsigned &status, int half = -1) {
   using R = typename std::conditional<MIXED, float, double>::type;
   constexpr int NQ = NComp<SHEAR, BULK>::value;
   const int o[5] = {(max(idx - 2, 0) - idx) * stride, (max(idx - 1, 0) - idx) * stride, 0,
@@ -307,6 +309,10 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
 
   R Sa[4];
   if (MIXED) axis_pi_sources<SHEAR, BULK, R>(a, s, axis, o, inv_d, uc, Sa);
+  auto add = [&](int n, R r) {
+    if (HALVES && half >= 0) reinterpret_cast<float *>(out + n * kBlock)[half] = (float)r;
+    else out[n * kBlock] += (double)r * dt;
+  };
   const R th = (R)a.theta;
   // the root-find components from the cache
   constexpr int NRC = 4 + (SHEAR ? 4 : 0) + (BULK ? 1 : 0);
@@ -317,7 +323,7 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
     R r = flux_from_states<R>((R)c[0], (R)c[kBlock], (R)c[2 * kBlock], (R)c[3 * kBlock], f);
     r = r * half_inv_d;
     if (SHEAR && MIXED && n < 4) r += Sa[n];
-    out[n * kBlock] += (double)r * dt;
+    add(n, r);
   }
   // pi^{ij} from the lattice, two components' stencil loads in flight at once (2 measured
   // faster than 1, 3 and 6)
@@ -330,7 +336,7 @@ __device__ __forceinline__ double axis_update(const StageArgs &a, int s, int axi
         const int m = spatial_of_pi(n, axis);
         if (m >= 0) out[(1 + m) * kBlock] -= ((double)centred * sink.fac) * sink.dt;
       }
-      out[n * kBlock] += (double)(r * half_inv_d) * dt;
+      add(n, r * half_inv_d);
     }
   }
   return fmax(fd.af, fd.ab);
@@ -647,7 +653,9 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_kernel(const 
 //              about the same time)
 // A part without the source term collects its components' increments (before the factor dt)
 // in its own shared-memory column; after a barrier part 0 adds them to its Euler update and
-// finishes the cell. The same functions as kt_stage_kernel, sums to rounding.
+// finishes the cell. The same functions as kt_stage_kernel; on the mixed path the same sums too, axis
+// by axis (PARTS = 2 keeps the y and the eta increment, floats, in the two halves of an element), in
+// FP64 to rounding.
 __host__ __device__ constexpr int split_cells(int parts) { return kBlock / parts; }
 static_assert(split_cells(4) % 32 == 0, "a part of a cell's stage is whole warps");
 
@@ -659,6 +667,7 @@ template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED, int PARTS>
 __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(const StageArgs a) {
   constexpr int NQ = NComp<SHEAR, BULK>::value;
   constexpr int kCells = split_cells(PARTS);
+  constexpr bool kHalves = MIXED && PARTS == 2;
   const int lane = threadIdx.x % kCells;
   const int part = threadIdx.x / kCells;
   const long long id = (long long)blockIdx.x * kCells + lane;
@@ -706,8 +715,10 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
       if (!MIXED && n_axis == 1) continue;
       const int stride = axis == 0 ? 1 : axis == 1 ? (int)a.sy : (int)a.sz;
       const double inv_spacing = axis == 0 ? a.inv_dx : axis == 1 ? a.inv_dy : a.inv_dz;
-      const double as = axis_update<EOS, SHEAR, BULK, MIXED>(a, (int)s, axis, idx, n_axis, stride, inv_spacing,
-                                                             part == 0 ? a.dt : 1.0, g0, uc, out, cache, status);
+      const double as =
+          axis_update<EOS, SHEAR, BULK, MIXED, kHalves>(a, (int)s, axis, idx, n_axis, stride, inv_spacing,
+                                                        part == 0 ? a.dt : 1.0, g0, uc, out, cache, status,
+                                                        part == 0 ? -1 : axis - 1);
       speed = fmax(speed, n_axis > 1 ? as * inv_spacing : 0.0);
     }
     if (part != 0 && status) atomicOr(a.status, status);
@@ -718,7 +729,15 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
     for (int p = 1; p < PARTS; ++p) {
       const double *inc = gvh_stage_smem + p * kCells + lane;
 #pragma unroll
-      for (int n = 0; n < NQ; ++n) out[n * kBlock] += inc[n * kBlock] * a.dt;
+      for (int n = 0; n < NQ; ++n) {
+        if (kHalves) {
+          const float2 r = reinterpret_cast<const float2 *>(inc)[n * kBlock];
+          out[n * kBlock] += (double)r.x * a.dt;
+          out[n * kBlock] += (double)r.y * a.dt;
+        } else {
+          out[n * kBlock] += inc[n * kBlock] * a.dt;
+        }
+      }
     }
     stage_finish<EOS, SHEAR, BULK, STAGE2, MIXED, kBlock>(a, s, out, guess_eos<EOS>(ePrev), status);
   }
