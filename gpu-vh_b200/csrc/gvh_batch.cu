@@ -33,7 +33,6 @@
 #include <vector>
 
 #include "../../include/gvh.h"
-#define GVH_BATCH_KERNELS  // bulk_zeta_over_s
 #include "gvh_layout.cuh"
 #include "gvh_nvtx.h"
 #include "gvh_stage.cuh"
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS)
     int i, j, k;
     double en = 0.0, speed;
     if (tile_cell(E, tile_x, tile - E.first_tile, threadIdx.x, i, j, k))
-      en = stage_cell_ijk<EOS, SHEAR, BULK, STAGE2, MIXED>(a, i, j, k, speed);
+      en = stage_cell_ijk<EOS, SHEAR, BULK, STAGE2, MIXED, true>(a, i, j, k, speed);
     if (STAGE2) {
       unsigned long long b = __double_as_longlong(fmax(en, 0.0));
 #pragma unroll

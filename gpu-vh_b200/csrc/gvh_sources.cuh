@@ -33,7 +33,8 @@ struct ShearT {
 // SourceTerms.cu:29-256. rhs[0..9] = d pi^{mu nu}/dtau (pitt..pinn), rhs[10] = dPi/dtau.
 // R = double reproduces the reference's FP64 arithmetic; R = float is the mixed path.
 // cs2_guess: c_s^2(e) from the cell's GuessEos (the FP64 path; the mixed path evaluates its own).
-template <int EOS, bool BULK, class R>
+// FUSED: zeta/s in single precision (bulk_zeta_over_s).
+template <int EOS, bool BULK, bool FUSED, class R>
 __device__ __forceinline__ void pimunu_rhs(R *rhs, R t, R etabar, R e, R p, const CellFlowT<R> &f,
                                            const ShearT<R> &pi, R Pi, R dkvk, double cs2_guess) {
   const R ut = f.ut, ux = f.ux, uy = f.uy, un = f.un;
@@ -179,7 +180,7 @@ __device__ __forceinline__ void pimunu_rhs(R *rhs, R t, R etabar, R e, R p, cons
     R a2 = a * a;
     R beta_Pi = R(15.0) * a2 * (e + p);
     R lambda_Pipi = R(kF16) * a;
-    R zetabar = bulk_zeta_over_s(T);
+    R zetabar = bulk_zeta_over_s<FUSED>(T);
     R tauPiInv = R(15) * a2 * dv(T, zetabar);
     R dPi = -beta_Pi * theta - Pi * tauPiInv - R(kDeltaBulk) * Pi * theta + lambda_Pipi * ps;
     rhs[10] = dPi * iut + Pi * dkvk;

@@ -361,7 +361,7 @@ constexpr size_t stage_smem_bytes() {
 // density so callers can reduce it (the batched engine tracks max e per event).
 // The source-term Euler step of one cell: out[n * OSTRIDE] = q_n + dt * S_n
 // (EulerStep.cu:946-1009, SourceTerms.cu:569-755).
-template <int EOS, bool SHEAR, bool BULK, bool MIXED, int OSTRIDE>
+template <int EOS, bool SHEAR, bool BULK, bool MIXED, int OSTRIDE, bool FUSED = false>
 __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, int i, int j, int k, double ePrev,
                                              const double (&uc)[4], const GuessEos &g0, double *out) {
   using R = typename std::conditional<MIXED, float, double>::type;
@@ -438,7 +438,7 @@ __device__ __forceinline__ void stage_source(const StageArgs &a, long long s, in
   if (SHEAR) {
     ShearT<R> pi{q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13]};
     R rhs[11];
-    pimunu_rhs<EOS, BULK, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk,
+    pimunu_rhs<EOS, BULK, FUSED, R>(rhs, t, (R)a.etabar, er, pc, f, pi, Pi, dkvk,
                               BULK && !MIXED ? guess_cs2<EOS>(g0) : 0.0);
 #pragma unroll
     for (int n = 4; n < NQ; ++n) S[n] = rhs[n - 4];
@@ -552,7 +552,7 @@ __host__ __device__ inline bool cell_stencil_ok(const StageArgs &a, int i, int j
 
 // speed: max over the axes with more than one cell of the local propagation speed over the lattice spacing,
 // a / dx_axis (the CFL bound of the step is dt times its maximum over cells).
-template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED>
+template <int EOS, bool SHEAR, bool BULK, bool STAGE2, bool MIXED, bool FUSED = false>
 __device__ __forceinline__ double stage_cell_ijk(const StageArgs &a, int i, int j, int k, double &speed) {
   using R = typename std::conditional<MIXED, float, double>::type;
   constexpr int NQ = NComp<SHEAR, BULK>::value;
@@ -579,7 +579,7 @@ __device__ __forceinline__ double stage_cell_ijk(const StageArgs &a, int i, int 
   double *cache = gvh_stage_smem + NQ * kBlock + threadIdx.x;
 
   const GuessEos g0 = guess_eos<EOS>(ePrev);
-  stage_source<EOS, SHEAR, BULK, MIXED, kBlock>(a, s, i, j, k, ePrev, uc, g0, out);
+  stage_source<EOS, SHEAR, BULK, MIXED, kBlock, FUSED>(a, s, i, j, k, ePrev, uc, g0, out);
 
   // ---- flux divergence along x, y, eta (EulerStep.cu:1011-1277) -------------------------
   speed = 0.0;
