@@ -18,7 +18,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
 #include <string>
 
 #include "../../include/gvh.h"
@@ -213,19 +212,11 @@ int gvh_create(const gvh_lattice_params *L, const gvh_hydro_params *H, const gvh
   int dev = o.device;
   if (dev < 0) GVH_CUDA(cudaGetDevice(&dev));
   GVH_CUDA(cudaSetDevice(dev));
-  {
-    // the stage kernels' shared-memory limit, once per device (kernel attributes are per device)
-    static std::mutex mu;
-    static unsigned long long prepared = 0;
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 64 && !(prepared & (1ull << dev))) {
-      GVH_CUDA(prepare_stage_kernels());
-      prepared |= 1ull << dev;
-    }
-  }
-
   int sms = 0;
   GVH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  GVH_CUDA(prepare_stage(o.eos, o.shear, o.bulk, o.precision,
+                         (long long)L->numLatticePointsX * L->numLatticePointsY * L->numLatticePointsRapidity,
+                         stage_wave_cells(sms)));
 
   gvh_handle *h = new gvh_handle();
   memset(h, 0, sizeof(*h));

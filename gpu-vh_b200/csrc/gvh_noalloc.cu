@@ -73,13 +73,13 @@ int scratch_address(int dev, unsigned char **out) {
       cudaError_t err = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_noalloc_scratch);
       if (err != cudaSuccess)
         return nfail(GVH_ERR_CUDA, "cudaGetSymbolAddress(scratch) on device %d: %s", dev, cudaGetErrorString(err));
-      // the stage kernels' shared-memory limit, part of the same one-time set-up
-      err = prepare_stage_kernels();
-      if (err != cudaSuccess)
-        return nfail(GVH_ERR_CUDA, "stage kernel set-up on device %d: %s", dev, cudaGetErrorString(err));
       int sms = 0;
       err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       if (err != cudaSuccess) return nfail(GVH_ERR_CUDA, "SM count of device %d: %s", dev, cudaGetErrorString(err));
+      // the stage kernels' shared-memory limit, part of the same one-time set-up
+      err = prepare_all_stages(stage_wave_cells(sms));
+      if (err != cudaSuccess)
+        return nfail(GVH_ERR_CUDA, "stage kernel set-up on device %d: %s", dev, cudaGetErrorString(err));
       g_wave_cells[dev] = stage_wave_cells(sms);
       g_scratch_ptr[dev].store(p, std::memory_order_release);
     }

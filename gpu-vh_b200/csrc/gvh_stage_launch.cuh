@@ -56,25 +56,27 @@ cudaError_t launch_stage_of(const StageArgs &a, int shear, int bulk, bool stage2
 }
 
 template <int EOS, bool MIXED, bool SHEAR, bool BULK, bool STAGE2>
-cudaError_t prepare_stage_kernel() {
+cudaError_t prepare_stage_kernel(int parts) {
   const size_t smem = stage_smem_bytes<SHEAR, BULK>();
-  cudaError_t e = allow_stage_smem(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, smem);
-  if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 2>, smem);
-  if (e == cudaSuccess) e = allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, smem);
-  if (e == cudaSuccess)
-    e = allow_stage_smem(kt_stage_faces_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, faces_smem_bytes<SHEAR, BULK>());
-  return e;
+  if (parts == 8)
+    return allow_stage_smem(kt_stage_faces_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, faces_smem_bytes<SHEAR, BULK>());
+  if (parts == 4) return allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 4>, smem);
+  if (parts == 2) return allow_stage_smem(kt_stage_split_kernel<EOS, SHEAR, BULK, STAGE2, MIXED, 2>, smem);
+  return allow_stage_smem(kt_stage_kernel<EOS, SHEAR, BULK, STAGE2, MIXED>, smem);
+}
+
+template <int EOS, bool MIXED, bool SHEAR, bool BULK>
+cudaError_t prepare_stage_physics(int parts) {
+  const cudaError_t e = prepare_stage_kernel<EOS, MIXED, SHEAR, BULK, false>(parts);
+  return e == cudaSuccess ? prepare_stage_kernel<EOS, MIXED, SHEAR, BULK, true>(parts) : e;
 }
 
 template <int EOS, bool MIXED>
-cudaError_t prepare_stages_of() {
-  cudaError_t e = prepare_stage_kernel<EOS, MIXED, false, false, false>();
-  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, false, false, true>();
-  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, false, false>();
-  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, false, true>();
-  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, true, false>();
-  if (e == cudaSuccess) e = prepare_stage_kernel<EOS, MIXED, true, true, true>();
-  return e;
+cudaError_t prepare_stage_of(int shear, int bulk, long long ncells, long long wave) {
+  const int parts = stage_parts(ncells, wave);
+  if (!shear) return prepare_stage_physics<EOS, MIXED, false, false>(parts);
+  if (!bulk) return prepare_stage_physics<EOS, MIXED, true, false>(parts);
+  return prepare_stage_physics<EOS, MIXED, true, true>(parts);
 }
 
 }  // namespace gvh

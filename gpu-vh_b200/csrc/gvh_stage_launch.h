@@ -11,17 +11,28 @@ namespace gvh {
 
 struct StageArgs;
 
-// Raises the stage kernels' shared-memory limits on the current device (once per device, before
-// any launch or capture).
-cudaError_t prepare_qcd_fp64();
-cudaError_t prepare_qcd_mixed();
-cudaError_t prepare_conformal_fp64();
-cudaError_t prepare_conformal_mixed();
-inline cudaError_t prepare_stage_kernels() {
-  cudaError_t e = prepare_qcd_fp64();
-  if (e == cudaSuccess) e = prepare_qcd_mixed();
-  if (e == cudaSuccess) e = prepare_conformal_fp64();
-  if (e == cudaSuccess) e = prepare_conformal_mixed();
+// Raises the shared-memory limit of the two stage kernels that a lattice of ncells takes on the
+// current device; before any launch or capture of them. Doing so loads a kernel (0.05 ms and 50 KB
+// of device memory each), so a handle prepares its own and not all 96.
+cudaError_t prepare_qcd_fp64(int shear, int bulk, long long ncells, long long wave);
+cudaError_t prepare_qcd_mixed(int shear, int bulk, long long ncells, long long wave);
+cudaError_t prepare_conformal_fp64(int shear, int bulk, long long ncells, long long wave);
+cudaError_t prepare_conformal_mixed(int shear, int bulk, long long ncells, long long wave);
+inline cudaError_t prepare_stage(int eos, int shear, int bulk, int precision, long long ncells, long long wave) {
+  const bool mixed = precision == GVH_PRECISION_MIXED;
+  if (eos == GVH_EOS_CONFORMAL)
+    return mixed ? prepare_conformal_mixed(shear, bulk, ncells, wave) : prepare_conformal_fp64(shear, bulk, ncells, wave);
+  return mixed ? prepare_qcd_mixed(shear, bulk, ncells, wave) : prepare_qcd_fp64(shear, bulk, ncells, wave);
+}
+// The same for every lattice (gvh_rk2_step_noalloc: its first call on a device is the only one that
+// may load kernels). The four sizes are one of each rule in stage_parts.
+inline cudaError_t prepare_all_stages(long long wave) {
+  cudaError_t e = cudaSuccess;
+  for (int eos : {GVH_EOS_QCD, GVH_EOS_CONFORMAL})
+    for (int precision : {GVH_PRECISION_FP64, GVH_PRECISION_MIXED})
+      for (int physics = 0; physics < 3; ++physics)  // ideal, shear, shear + bulk
+        for (long long ncells : {wave / 8, wave / 4, wave / 2, wave})
+          if (e == cudaSuccess) e = prepare_stage(eos, physics > 0, physics > 1, precision, ncells, wave);
   return e;
 }
 
