@@ -345,7 +345,7 @@ int pinned_mark(gvh_batch *b, PinnedBuf &p) {
 // The tile -> event table of the admitted events (each event's tiles contiguous, events in
 // slot order) and its count go to the device through a pinned buffer; first_tile of every
 // event is derived on the device. Nothing waits for the device; a tile count that changes under a
-// one-block-per-tile grid leaves the step's graph stale until the next step (step_graph).
+// one-block-per-tile grid leaves the step's graph stale until the next step (queue_steps).
 int rebuild_tiles(gvh_batch *b) {
   int slots = 0, n = 0;
   for (size_t i = 0; i < b->ev.size(); ++i)

@@ -755,8 +755,8 @@ __global__ void __launch_bounds__(kBlock, GVH_MIN_BLOCKS) kt_stage_split_kernel(
 // a block of eight warps takes 32 cells: warp 0 their source terms, warps 1..6 one face of one
 // axis each (two recoveries, fifteen fluxes), warp 7 the axes' pi, Pi derivative sources. After a
 // barrier the eight warps share the components of the Euler update (and the Heun combination),
-// then warp 0 finishes the cells. The expressions of kt_stage_kernel's mixed path bit for bit, of
-// its FP64 path to rounding.
+// then warp 0 finishes the cells. The sums of kt_stage_kernel on the mixed path, bit for bit, in FP64 to
+// rounding (tests/test_stage_parts_gpu.py).
 constexpr int kFaceBlock = 256;
 constexpr int kFaceCells = 32;
 
