@@ -705,22 +705,25 @@ def run_ours(args):
     achieved = cells * b_cell / (ms / args.steps / 1e3) / 1e9
     traffic = None
     fp64_pipe = None
+    counters_of = None
     tp = os.path.join(ROOT, "profiles", "kt_stage_traffic.json")
     if os.path.exists(tp):
         try:
             prof = json.load(open(tp))
             traffic = prof.get("bytes_per_step")
             fp64_pipe = prof.get("fp64_pipe_active_pct")
+            counters_of = prof.get("build")
         except Exception:
             traffic = None
     # One step is the kernel's two launches (stage 1 + stage 2): achieved, traffic and the
-    # algorithmic bytes are all per step. The kernel's real limit is FP64 issue, so the FP64
-    # pipe's busy fraction from the same capture is given beside the HBM roofline.
+    # algorithmic bytes are all per step. The kernel's real limit is the latency of dependent FP64
+    # operations, so the FP64 pipe's busy fraction is given beside the HBM roofline. traffic and that
+    # fraction are read from a profiler's capture, of the build named beside them, not of this run.
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "peak_source": peak_kind,
                 "algorithmic_bytes_per_step": cells * b_cell,
                 "per": "step (2 launches of kt_stage_kernel)",
-                "fp64_pipe_active_pct": fp64_pipe,
+                "fp64_pipe_active_pct": fp64_pipe, "counters_of_build": counters_of,
                 "kernel": "kt_stage_kernel (stage 1 + stage 2 per step)"}
 
     extras = {}
